@@ -164,29 +164,23 @@ typedef struct {
                                       a launch).  Same results; needs imaging_period 1 for the Hessian */
     int forward_only;              /* 1 = only forward modelling (pysit_plan_forward): no adjoint,
                                       checkpoint or imaging buffers; other runs return PYSIT_EINVAL */
-    double shell_share[3];         /* 2D, per step mode (forward, recompute, adjoint): share of the GPU's
-                                      resident blocks given to the PML-shell kernel, in (0, 1), so that it
-                                      runs beside the interior kernel from the start; 0 = each kernel sized
-                                      for the whole GPU (the default: inside the CUDA graph of a sweep
-                                      that balanced the two kernels best in measurements) */
+    double shell_share[3];         /* kept for callers of an earlier step of two kernels: in (0, 1) per
+                                      step mode; read back by pysit_plan_get_tuning, without effect
+                                      (the 2D step is one kernel over interior and PML-shell tiles) */
     int lanes;                     /* >= 2: the shots are split into that many contiguous ranges whose
                                       launch sequences run side by side on their own streams (each lane
                                       with its own buffers: lanes x the workspace of its shots); 0 or 1 =
                                       one sequence.  Results are the lanes' sums, in lane order */
-    uint32_t wait_polls;           /* 0 = a step kernel's wait for a bulk copy into shared memory makes
-                                      up to 2^22 blocking tries (far beyond any copy's latency); n > 0 =
-                                      at most n non-blocking tests before the wait counts as expired.
-                                      An expired wait sets bit 0 of the status word; the warp waits
-                                      (with the full limit) for the copies it has in flight and runs
-                                      no further task, so the run's results are invalid */
-    int wait_fault;                /* test aid, 0 in normal use.  1 = every task of the 2D step kernels
-                                      first waits (bounded: wait_polls non-blocking tests, 64 when
-                                      wait_polls is 0) on an mbarrier on which nothing ever arrives;
-                                      the wait runs out and takes the expiry path above with the
-                                      task's bulk copies in flight.  Lets a test check that path and
-                                      the status report without any GPU fault */
+    uint32_t wait_polls;           /* non-blocking tests of the wait that wait_fault adds (0: 64); the
+                                      step kernels have no other device wait */
+    int wait_fault;                /* test aid, 0 in normal use.  1 = every block of the 2D step kernels
+                                      first waits (bounded: wait_polls non-blocking tests) on an
+                                      mbarrier on which nothing ever arrives; the wait runs out, the
+                                      block sets bit 0 of the status word and leaves its tile undone, so
+                                      the run's results are invalid.  Lets a test check the status
+                                      report without any GPU fault */
     int tile_z;                    /* 2D/3D: z extent of an interior task at most, in cells (a multiple of
-                                      4, >= 16); 0 = the kernel's full width (32 lanes x the lane vector:
+                                      4, >= 16); 0 = the kernel's full width (32 threads x their vector:
                                       128 cells in FP32, 64 in FP64).  Narrower tasks leave lanes idle but
                                       make more tasks; pysit_plan_autotune_tiles chooses it by timing */
 } pysit_plan_desc;
@@ -242,7 +236,7 @@ int pysit_plan_born(pysit_plan* plan, const double* m1_dev, void* traces_dev, vo
 int pysit_plan_hessian(pysit_plan* plan, const double* m1_dev, double* out_dev, double* d1norm2_dev,
                        void* stream);
 /* Reads and clears the plan's device status word (synchronises `stream`):
- * bit 0 (1) = a bounded wait for a bulk copy expired (results invalid),
+ * bit 0 (1) = a bounded device wait expired (results invalid),
  * bit 1 (2) = a non-finite wavefield value appeared (unstable time step). */
 int pysit_plan_status(pysit_plan* plan, int* flags, void* stream);
 /* ------------------------------------------------------------------------
@@ -296,7 +290,7 @@ int pysit_plan_autotune_tiles(pysit_plan* plan, const int* cand_x, int ncx, cons
 int pysit_plan_get_tiles(const pysit_plan* plan, int* tile_x, int* tile_z);
 /* A host copy of the plan's current task table, no counterpart in the reference (diagnostics
  * and tests; needs no device).  2D: rows of 5 ints (x0, x1, zs, ze, kind: 0 interior, 1 PML
- * shell), the warp tasks of one shot; 3D: rows of 6 ints (x0, x1, y0, y1, zs, ze), one block of
+ * shell), the tiles of one shot; 3D: rows of 6 ints (x0, x1, y0, y1, zs, ze), one block of
  * 8 warps each, a warp taking 32 / ceil((ze - zs) / V) y-rows (V = 4 FP32, 2 FP64 cells a lane);
  * 1D: none.  The interior tasks come first, *n_interior of them.  *n_ints receives the table's
  * size in ints; at most cap ints are written to out (which may be NULL). */

@@ -32,10 +32,6 @@
 
 #include "wave.cuh"
 
-#ifndef PGB_REC_BLOCKS_PER_SM
-#define PGB_REC_BLOCKS_PER_SM 1  // 2D recorder blocks per SM (leading blocks of the interior kernel)
-#endif
-
 namespace pgb {
 namespace {
 
@@ -75,34 +71,13 @@ __global__ void set_c2_kernel(const double* __restrict__ C, int nx, int ny, int 
     }
 }
 
-// Injection term of one 2D step added after the stencil kernels:
-//     u_{k+1} += fac C^2 rhs,   fac = dt^2, or 2 dt^2 / (2 + dt (sx + sz)) where a sigma is nonzero,
-// the factor the reference's update applies to C^2 (rhs + ...) (_2D.h:157-179); the update is
+// Injection term of one 3D step added after the stencil kernels:
+//     u_{k+1} += fac C^2 rhs,   fac = dt^2, or 2 dt^2 / (2 + dt (sx + sy + sz)) where a sigma is nonzero,
+// the factor the reference's update applies to C^2 (rhs + ...) (_3D.h:220-226); the update is
 // linear in rhs, so adding it afterwards equals injecting it inside the stencil.  One thread per
 // (shot, cell of the shot's injection box); cells of the outer ring are left alone, as the
 // reference skips them.  Used for wide operators (the adjoint source at every receiver), whose
 // per-cell tap walk would stall the stencil's row loop.
-template <typename T>
-__global__ void inject_scatter2d_kernel(const WaveParams<T> p, int cells_max) {
-    const long long n = (long long)p.nshot * cells_max;
-    for (long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x; id < n;
-         id += (long long)gridDim.x * blockDim.x) {
-        const int shot = (int)(id / cells_max), c = (int)(id - (long long)shot * cells_max);
-        const int* bx = p.inj.box + shot * 6;
-        const int bzw = bx[5] - bx[4];
-        if (bzw <= 0 || c >= (bx[1] - bx[0]) * bzw) continue;
-        const int x = bx[0] + c / bzw, z = bx[4] + c % bzw;
-        if (x <= 0 || x >= p.nx - 1 || z <= 0 || z >= p.nz - 1) continue;
-        const T rhs = inject_rhs(p.inj, bx, shot, x, z);
-        const T sx = p.sgx[x], sz = p.sgz[z];
-        const T fac = (sx != T(0) || sz != T(0)) ? T(2) * p.dt2 / (T(2) + p.dt * (sx + sz)) : p.dt2;
-        const long long o = foff2(p, x, z);
-        p.u_prev[(long long)shot * p.fstride + o] += fac * p.c2[o] * rhs;
-    }
-}
-
-// The same for a 3D step: fac = 2 dt^2 / (2 + dt (sx + sy + sz)) where a sigma is
-// nonzero (_3D.h:220-226).
 template <typename T>
 __global__ void inject_scatter3d_kernel(const WaveParams<T> p, int cells_max) {
     const long long n = (long long)p.nshot * cells_max;
@@ -132,7 +107,7 @@ __global__ void inject_scatter3d_kernel(const WaveParams<T> p, int cells_max) {
 // Born source of one step added after the stencil kernels of the scattered field u1:
 //     u1_{k+1} += fac C^2 rhs1,   rhs1 = -m1 dWaveOp0_k
 // (TemporalModeling.linear_forward_model, pysit/modeling/temporal_modeling.py:520-525; the
-// step is linear in rhs, fac as in inject_scatter2d/3d_kernel).  One block per row
+// step is linear in rhs, fac as in inject_scatter3d_kernel).  One block per row
 // (shot, x, y) of the padded grid, threads along z; cells of the outer ring are skipped as
 // the reference's step skips them.  m1 and C^2 are shared by the shots; dw holds dWaveOp0_k
 // of every shot of the launch.
@@ -177,9 +152,11 @@ __global__ void edge_pad_kernel(const double* __restrict__ m, int nx, int ny, in
 }
 
 // trace recorder as a kernel of its own (runs beside the stencil kernels: it only reads u_k)
+constexpr int kRecThreads = 128;
 template <typename T>
-__global__ void record_kernel(const WaveParams<T> p) {
-    record_block(p, blockIdx.x);
+__global__ void __launch_bounds__(kRecThreads) record_kernel(const WaveParams<T> p) {
+    const long long pass = (long long)blockIdx.x * (kRecThreads / 32) + (threadIdx.x >> 5);
+    if (pass < record_passes(p)) record_pass(p, pass);
 }
 
 constexpr int kRedBlocks = 1024;
@@ -333,8 +310,8 @@ struct PlanT final : public pysit_plan {
     int nslots = 1;              // replay slots: S (checkpointed) or ceil(nsteps / p_img) (kept)
     int tile_req = 0;            // requested task length along x (0: default)
     int tz = 0;                  // z extent of an interior task at most (0: the kernel's full width)
-    unsigned wait_polls = 0;     // tries of a step kernel's bulk-copy wait (0: the kernels' default)
-    int wait_fault = 0;          // test aid: the 2D step kernels' waits run out (pysit_plan_desc.wait_fault)
+    unsigned wait_polls = 0;     // tests of the wait that wait_fault adds (pysit_plan_desc.wait_polls)
+    int wait_fault = 0;          // test aid: a wait of the 2D step kernels runs out (pysit_plan_desc.wait_fault)
     std::vector<int> shot_steps; // record length of each shot in steps (empty: all nsteps)
     size_t task_cap = 0;         // ints the task buffer holds (enough for any tile the tuner may set)
     double dx, dy, dz, dt;
@@ -346,24 +323,21 @@ struct PlanT final : public pysit_plan {
     long long fstride;  // elements per field per shot (256-byte multiple)
     int bz, tx, ntz, ntx;
     int nseg;
-    std::vector<int> tasks2d;    // [ntasks][5] warp tasks of the 2D sweep: interior first, then shell
+    std::vector<int> tasks2d;    // [ntasks][5] tiles of the 2D step: interior first, then shell
     int ntask2d[2] = {0, 0};     // tasks of each kind
     std::vector<int> tasks3d;    // [ntasks][6] block tasks of the 3D sweep: interior first, then shell
     int ntask3d[2] = {0, 0};
-    int blocks2d[4][2] = {{1, 1}, {1, 1}, {1, 1}, {1, 1}};  // resident task blocks per mode and kind (whole GPU)
-    unsigned long long ctr_next[2] = {0, 0};  // task-counter values the next 2D launch starts at
-    double shell_frac[4] = {0.0, 0.0, 0.0, 0.0};  // 2D, per mode: share of the resident blocks given to the
-                                 // PML-shell kernel (0: each kernel is sized for the whole GPU and they
-                                 // overlap only where one runs out)
-    cudaStream_t aux = nullptr;  // second stream of the 2D step (shell kernel beside the interior one)
+    int strip2d = 4;             // 2D: x-rows per thread of a tile
+    std::vector<Tile2d> tiles2d;      // 2D: the device's form of tasks2d
+    int inj_cap[2] = {0, 0};     // 2D: injection cells of a tile at most (source, receivers)
+    double shell_frac[4] = {0.0, 0.0, 0.0, 0.0};  // descriptor's shell shares (read back by tuning(); unused)
+    cudaStream_t aux = nullptr;  // second stream of the 3D step (shell kernel beside the interior one)
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     // ---- acquisition (host) ----------------------------------------------------
     std::vector<CSRBox> src_inj, rec_inj;
     int rec_box_max = 0;              // largest receiver injection box (cells) over the shots
-    bool rec_in_shell = false;        // 2D: every receiver box lies in cells of PML-shell tasks only
     std::vector<int> rec_rows;        // [nshots*nrec+1]
     int rec_lanes = 1;                // recorder threads per (shot, receiver)
-    mutable int rec_cap = 0;          // 2D: recorder blocks at most (a share of the block slots; 0: not yet known)
     std::vector<long long> rec_off;   // internal offsets
     std::vector<double> rec_ws;       // sampling weights
     std::vector<double> src_amp;      // [nshots][nsteps][nsrc]
@@ -378,7 +352,7 @@ struct PlanT final : public pysit_plan {
         size_t sbox, srpb, srow, spt, sw;          // source injection
         size_t rbox, rrpb, rrow, rpt, rw;          // receiver injection
         size_t recrow, recoff, recw;               // recording
-        size_t gpad, partial, rnorm, err, tasks, ctr, shsteps;
+        size_t gpad, partial, rnorm, err, tasks, shsteps;
     } off{};
     size_t field_bytes = 0;      // one field for G shots
     int ckpt_fields = 0;         // fields per checkpoint
@@ -490,17 +464,7 @@ struct PlanT final : public pysit_plan {
         rec_box_max = 0;
         for (auto& b : rec_inj)
             rec_box_max = std::max(rec_box_max, (b.box[1] - b.box[0]) * (b.box[3] - b.box[2]) * (b.box[5] - b.box[4]));
-        if (dim == 2) {
-            // the bounds of the interior tasks (as build_tasks2d_ draws them)
-            const int xa = pl[0] > 0 ? pl[0] + R : 1, xb = pr[0] > 0 ? nx - pr[0] - R : nx - 1;
-            const int za = ((pl[2] > 0 ? pl[2] + R : 1) + 3) / 4 * 4, zb = (pr[2] > 0 ? nz - pr[2] - R : nz - 1) / 4 * 4;
-            rec_in_shell = !rec_inj.empty();
-            for (auto& b : rec_inj) {
-                if (b.box[1] <= b.box[0] || b.box[5] <= b.box[4]) continue;  // no taps
-                const bool zout = b.box[5] <= za || b.box[4] >= zb, xout = b.box[1] <= xa || b.box[0] >= xb;
-                if (!(zout || xout || xa >= xb || za >= zb)) rec_in_shell = false;
-            }
-        }
+        if (dim == 2) size_tiles2d();
         rc = build_recording(d);
         if (rc) return rc;
         src_amp.assign(d.src_amp, d.src_amp + (size_t)nshots * nsteps * nsrc);
@@ -511,8 +475,9 @@ struct PlanT final : public pysit_plan {
     void choose_tiling() {
         constexpr int V = V16<T>::N;
         if (dim == 2) {
-            bz = wave2d_warp_threads();
+            bz = kT2;
             tx = tile_req ? tile_req : 32;
+            strip2d = choose_strip2d();
             build_tasks2d();
             ntz = ntx = 1;
             return;
@@ -536,9 +501,20 @@ struct PlanT final : public pysit_plan {
         ntx = (nx + tx - 1) / tx;
     }
 
-    // Warp tasks covering the padded grid once.  Interior (kind 0): cells at least
+    // x-rows per thread of the 2D tiles.  Four rows share the most loads, but make the fewest
+    // threads: a launch too small to give every SM its resident blocks at four rows takes two, and
+    // one below that.  Measured (us per step at 4 / 2 / 1 rows): FP32 1232 x 464 x 64 shots 162 / 209
+    // / 236, x 4 13.0 / 14.0 / 16.0, x 1 (279 blocks at four rows) 5.9 / 5.4 / 5.4; FP64 461 x 203 x 6
+    // (548) 92 / 78 / 80; FP64 141 x 81 x 1 (11) 21 / 12.5 / 7.8
+    int choose_strip2d() const {
+        const long long threads = (long long)nx * nz * G / (16 / (int)sizeof(T));
+        const int full = 4 * 152;  // resident blocks of the GPU
+        return threads >= 4LL * kT2 * full ? 4 : threads >= 2LL * kT2 * full / 2 ? 2 : 1;
+    }
+
+    // Tiles covering the padded grid once.  Interior (kind 0): cells at least
     // R away from the padding; PML shell (kind 1): the rest.  z boundaries are
-    // multiples of 4 cells (vectors never straddle two tasks) except the grid end.
+    // multiples of 4 cells (vectors never straddle two tiles) except the grid end.
     void split(int a, int b, int w, std::vector<std::pair<int, int>>& out) const {
         if (b <= a) return;
         int n = (b - a + w - 1) / w;
@@ -569,10 +545,16 @@ struct PlanT final : public pysit_plan {
     void add_tasks(int xa, int xb, int za, int zb, int kind) {
         if (xb <= xa || zb <= za) return;
         std::vector<std::pair<int, int>> zs;
-        int w = wave2d_warp_seg((int)sizeof(T), order, kind);
+        int w = wave2d_seg((int)sizeof(T), kind);
         if (kind == 0 && tz > 0) w = std::min(w, tz);
         split(za, zb, w, zs);
-        const int nxc = (xb - xa + tx - 1) / tx, wx = (xb - xa + nxc - 1) / nxc;  // even x chunks
+        // even x chunks of at most tx rows, whole rounds of the block's strips
+        int zw = 0;
+        for (auto& z : zs) zw = std::max(zw, z.second - z.first);
+        const int once = wave2d_tile_rows((int)sizeof(T), kind, strip2d, zw);
+        const int rows = std::min(once, tx);
+        const int nxc = (xb - xa + rows - 1) / rows;
+        const int wx = std::min(rows, ((xb - xa + nxc - 1) / nxc + strip2d - 1) / strip2d * strip2d);
         for (int x = xa; x < xb; x += wx)
             for (auto& z : zs) {
                 int t[5] = {x, std::min(xb, x + wx), z.first, z.second, kind};
@@ -585,6 +567,30 @@ struct PlanT final : public pysit_plan {
         // interior tasks were added first
         ntask2d[0] = ntask2d[1] = 0;
         for (size_t t = 0; t < tasks2d.size(); t += 5) ++ntask2d[tasks2d[t + 4] ? 1 : 0];
+        size_tiles2d();
+    }
+    // injection cells of the largest tile's part of any shot's box, and the shared memory of a block
+    void size_tiles2d() {
+        auto cells = [&](const std::vector<CSRBox>& v) {
+            long long most = 0;
+            for (auto& b : v) {
+                if (b.box[1] <= b.box[0] || b.box[5] <= b.box[4]) continue;  // no taps
+                for (size_t t = 0; t < tasks2d.size(); t += 5) {
+                    const long long dx = std::min(b.box[1], tasks2d[t + 1]) - std::max(b.box[0], tasks2d[t]);
+                    const long long dz = std::min(b.box[5], tasks2d[t + 3]) - std::max(b.box[4], tasks2d[t + 2]);
+                    if (dx > 0 && dz > 0) most = std::max(most, dx * dz);
+                }
+            }
+            return (int)((most + 3) / 4 * 4);
+        };
+        inj_cap[0] = cells(src_inj);
+        inj_cap[1] = cells(rec_inj);
+        tiles2d.clear();
+        for (size_t t = 0; t < tasks2d.size(); t += 5) {
+            const int rows = tasks2d[t + 1] - tasks2d[t], nc = tasks2d[t + 3] - tasks2d[t + 2], kind = tasks2d[t + 4];
+            const int V = wave2d_cells((int)sizeof(T), kind), nzv = (nc + V - 1) / V;
+            tiles2d.push_back({tasks2d[t], rows, tasks2d[t + 2], nc, nzv, (65536 + nzv - 1) / nzv, kind, 0});
+        }
     }
     void build_tasks2d_() {
         // interior: R cells clear of the padding and off the outer (Dirichlet) ring
@@ -790,14 +796,13 @@ struct PlanT final : public pysit_plan {
         off.recw = take(std::max<size_t>(rec_ws.size(), 1) * sizeof(T));
         off.gpad = take((size_t)nx * ny * nz * sizeof(double));
         off.err = take(sizeof(int));
-        off.ctr = take(2 * sizeof(unsigned long long));
         off.shsteps = take(std::max<size_t>(shot_steps.size(), 1) * sizeof(int));
         // the largest table any tuning can ask for: the shortest x-chunk, and every z extent
         // (in 3D a narrower segment can give more tasks: its warps take several rows, but
         // not always enough to make up for the extra segments)
         task_cap = std::max<size_t>(task_ints(kMinTileX, 0), std::max(tasks2d.size(), tasks3d.size()));
         for (int z = kMinTileZ; z <= 32 * V16<T>::N; z += 4) task_cap = std::max(task_cap, task_ints(kMinTileX, z));
-        off.tasks = take(std::max<size_t>(task_cap, 1) * sizeof(int));
+        off.tasks = take(std::max<size_t>(dim == 2 ? task_cap / 5 * sizeof(Tile2d) : task_cap * sizeof(int), sizeof(Tile2d)));
         off.partial = take(kRedBlocks * sizeof(double));
         off.rnorm = take(sizeof(double));
         ws_need = tot;
@@ -860,16 +865,11 @@ struct PlanT final : public pysit_plan {
         if ((rc = upload_inj(rec_inj, off.rbox, off.rrpb, off.rrow, off.rpt, off.rw, s))) return rc;
         if ((rc = upload(off.recrow, rec_rows, s)) || (rc = upload(off.recoff, rec_off, s))) return rc;
         if ((rc = upload(off.recw, tmp = toT(rec_ws), s))) return rc;
-        if ((rc = upload(off.tasks, dim == 3 ? tasks3d : tasks2d, s))) return rc;
+        if ((rc = dim == 3 ? upload(off.tasks, tasks3d, s) : upload(off.tasks, tiles2d, s))) return rc;
         if ((rc = upload(off.shsteps, shot_steps, s))) return rc;
         PGB_CHECK_CUDA(cudaStreamSynchronize(s));
         if (!cap) PGB_CHECK_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
-        if (dim == 2) {
-            wave2d_warp_prepare();
-            for (int m = 0; m < 4; ++m)
-                for (int k = 0; k < 2; ++k) blocks2d[m][k] = wave2d_warp_blocks((int)sizeof(T), order, m, k);
-        }
-        if (dim >= 2) {
+        if (dim == 3) {
             if (!aux) PGB_CHECK_CUDA(cudaStreamCreateWithFlags(&aux, cudaStreamNonBlocking));
             if (!ev_fork) PGB_CHECK_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
             if (!ev_join) PGB_CHECK_CUDA(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
@@ -921,7 +921,6 @@ struct PlanT final : public pysit_plan {
         p.polls = wait_polls;
         p.wait_fault = wait_fault;
         p.psi_c2 = psi_consistent ? 0 : 1;
-        p.task_ctr = ws ? at<unsigned long long>(off.ctr) : nullptr;
         (void)g0;
         return p;
     }
@@ -949,76 +948,18 @@ struct PlanT final : public pysit_plan {
         }
     }
 
-    // One 2D step: the interior kernel on s and the PML-shell kernel on the
-    // auxiliary stream, forked from and joined back into s (graph branches when
-    // captured), each a persistent grid drawing (shot, task) pairs from its counter.
+    // One 2D step: one launch over the tiles of every shot (the traces recorded and the
+    // injection worked out by the blocks' producer warps).
     template <int RR, int MODE>
     void launch2d(const WaveParams<T>& p, cudaStream_t s) {
-        const int* tk = at<int>(off.tasks);
-        const long long wpb = wave2d_warp_threads() / 32;
         WaveParams<T> q = p;
-        q.task_base = ctr_next[0];
-        q.task_base2 = ctr_next[1];
-        int nb[2];
-        // with a shell share the two kernels split the resident block slots (they run side by
-        // side from the start); otherwise each is sized for the whole GPU
-        const double fr = shell_frac[MODE];
-        const int cap1 = fr > 0 ? std::max(1, (int)(fr * blocks2d[MODE][1] + 0.5)) : blocks2d[MODE][1];
-        const int cap0 = fr > 0 ? std::max(1, blocks2d[MODE][0] - (int)(fr * blocks2d[MODE][0] + 0.5))
-                                : blocks2d[MODE][0];
-        for (int k = 0; k < 2; ++k) {
-            const long long need = ((long long)ntask2d[k] * p.nshot + wpb - 1) / wpb;
-            nb[k] = (int)std::min<long long>(need, k ? cap1 : cap0);
-        }
-        // the adjoint source covers every receiver: added by a scatter kernel after the step
-        const bool scatter = MODE == kAdj && q.inj.on && rec_box_max > 0;
-        if (scatter) q.inj.on = 0;
-        const bool rec = MODE != kAdj && q.rec.blocks > 0;
-        const int recb = q.rec.blocks;
-        q.rec.blocks = 0;
-        const bool fork = ntask2d[1] > 0 && ntask2d[0] > 0;
-        cudaStream_t side = fork ? aux : s;
-        if (fork) {
-            cudaEventRecord(ev_fork, s);
-            cudaStreamWaitEvent(aux, ev_fork, 0);
-        }
-#ifndef PGB_FUSED_REC
-#define PGB_FUSED_REC 1
-#endif
-        // the recorder rides as extra leading blocks of the interior kernel (they read u_k,
-        // which the step leaves alone, and exit at once); as a kernel of its own ahead of the
-        // shell kernel it held the shell back until the interior kernel's blocks retired
-        const bool fused_rec = PGB_FUSED_REC && rec && ntask2d[0] > 0;
-        if (rec && !fused_rec) {
-            record_kernel<T><<<recb, bz, 0, side>>>(q);
-            ++launches;
-        }
-        if (ntask2d[1] > 0) {
-            ctr_next[1] += launch_wave2d_warp_tasks<T, RR, MODE, 1>(q, tk + 5 * ntask2d[0], ntask2d[1], nb[1], side);
-            ++launches;
-        }
-        if (ntask2d[0] > 0) {
-            WaveParams<T> qi = q;
-            qi.rec.blocks = fused_rec ? recb : 0;
-            ctr_next[0] += launch_wave2d_warp_tasks<T, RR, MODE, 0>(qi, tk, ntask2d[0], nb[0], s);
-            ++launches;
-        }
-        // the adjoint source adds to cells the shell kernel has written; when every receiver
-        // box lies in shell cells it follows the shell kernel on its stream, overlapping the
-        // interior kernel's tail, else it waits for both
-        const bool scatter_side = scatter && fork && rec_in_shell;
-        auto do_scatter = [&](cudaStream_t st) {
-            q.inj.on = 1;
-            const long long n = (long long)q.nshot * rec_box_max;
-            inject_scatter2d_kernel<T><<<(int)std::min<long long>((n + 255) / 256, 4096), 256, 0, st>>>(q, rec_box_max);
-            ++launches;
-        };
-        if (scatter_side) do_scatter(side);
-        if (fork) {
-            cudaEventRecord(ev_join, aux);
-            cudaStreamWaitEvent(s, ev_join, 0);
-        }
-        if (scatter && !scatter_side) do_scatter(s);
+        // a launch whose wavefields exceed L2 (126 MB): a block fetches the next shot's tile.
+        // 64 shots of 1232 x 464 cells (FP32): recompute 175 -> 162, adjoint 248 -> 215 us; two or
+        // three shots ahead 162 / 166 and 230 / 257 us
+        q.pf_next = p.nshot > 1 && 2 * (size_t)fstride * sizeof(T) * p.nshot > ((size_t)48 << 20);
+        launch_wave2d_tiles<T, RR, MODE>(q, at<Tile2d>(off.tasks), ntask2d[0], ntask2d[1], strip2d,
+                                         inj_cap[MODE == kAdj], s);
+        ++launches;
     }
 
     // One 3D step: interior kernel on s, PML-shell kernel (and the trace recorder)
@@ -1030,7 +971,7 @@ struct PlanT final : public pysit_plan {
         WaveParams<T> q = p;
         const bool scatter = MODE == kAdj && q.inj.on && rec_box_max > 0;
         if (scatter) q.inj.on = 0;
-        const bool rec = MODE != kAdj && q.rec.blocks > 0;
+        const bool rec = MODE != kAdj && q.rec.traces && q.rec.nrec > 0;
         const bool fork = ntask3d[0] > 0 && (ntask3d[1] > 0 || rec);
         cudaStream_t side = fork ? aux : s;
         if (fork) {
@@ -1038,7 +979,8 @@ struct PlanT final : public pysit_plan {
             cudaStreamWaitEvent(aux, ev_fork, 0);
         }
         if (rec) {
-            record_kernel<T><<<q.rec.blocks, bz, 0, side>>>(q);
+            const long long passes = ((long long)q.nshot * q.rec.nrec * q.rec.lanes + 31) / 32;
+            record_kernel<T><<<(int)((passes * 32 + kRecThreads - 1) / kRecThreads), kRecThreads, 0, side>>>(q);
             ++launches;
         }
         if (ntask3d[1] > 0) {
@@ -1280,7 +1222,6 @@ struct PlanT final : public pysit_plan {
     }
 
     void enqueue_born(const double* m1, void* traces_out, cudaStream_t s) {
-        reset_task_counter(s);
         pad_perturbation(m1, s);
         const size_t tr_group = (size_t)nsteps * nrec * sizeof(T);
         for (int g0 = 0; g0 < nshots; g0 += G) {
@@ -1296,7 +1237,6 @@ struct PlanT final : public pysit_plan {
     // checkpoints the Born sweep saved (apply_hessian 'approximate',
     // temporal_least_squares.py:209-217; migrate_shot images every step)
     void enqueue_hessian(const double* m1, double* out, double* d1norm2, cudaStream_t s) {
-        reset_task_counter(s);
         pad_perturbation(m1, s);
         cudaMemsetAsync(ws + off.gpad, 0, (size_t)nx * ny * nz * sizeof(double), s);
         cudaMemsetAsync(ws + off.rnorm, 0, sizeof(double), s);
@@ -1345,12 +1285,6 @@ struct PlanT final : public pysit_plan {
                    [&](cudaStream_t st) { enqueue_hessian(m1, out, d1norm2, st); });
     }
 
-    // the 2D sweep's task counter restarts at zero with every run (eager or graph replay)
-    void reset_task_counter(cudaStream_t s) {
-        cudaMemsetAsync(ws + off.ctr, 0, 2 * sizeof(unsigned long long), s);
-        ctr_next[0] = ctr_next[1] = 0;
-    }
-
     // n launches of one step kernel on the first shot group's buffers, for timing
     // (the state keeps evolving from whatever the last run left; no output)
     int step_loop(int mode, int n, cudaStream_t s) override {
@@ -1360,7 +1294,6 @@ struct PlanT final : public pysit_plan {
         PGB_REQUIRE(!fwd_only || mode == kFwd, "the plan was built for forward modelling only");
         PGB_REQUIRE(n >= 0, "nsteps must be >= 0");
         launches = 0;
-        reset_task_counter(s);
         const int gn = std::min(G, nshots);
         WaveParams<T> p = base_params(0, gn);
         State st = mode == kAdj ? make_state(off.A, off.AX, off.AY, off.AZ, off.AS)
@@ -1472,7 +1405,8 @@ struct PlanT final : public pysit_plan {
         tz = z > 0 ? z / 4 * 4 : 0;
         std::vector<int>& tab = dim == 3 ? (build_tasks3d(), tasks3d) : (build_tasks2d(), tasks2d);
         PGB_REQUIRE(tab.size() <= task_cap, "task table of %zu ints exceeds its buffer (%zu)", tab.size(), task_cap);
-        PGB_CHECK_CUDA(cudaMemcpyAsync(ws + off.tasks, tab.data(), tab.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+        int rc = dim == 3 ? upload(off.tasks, tasks3d, s) : upload(off.tasks, tiles2d, s);
+        if (rc) return rc;
         PGB_CHECK_CUDA(cudaStreamSynchronize(s));
         for (auto& kv : graphs)
             if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
@@ -1489,24 +1423,9 @@ struct PlanT final : public pysit_plan {
         p.rec.tr_sstride = (long long)nsteps * nrec;
         p.rec.nrec = nrec;
         p.rec.lanes = rec_lanes;
-        // 2D: the recorder blocks lead the interior kernel's grid and hold one of its block
-        // slots each while they run, so a few of them stride over the receivers and the step's
-        // own blocks take the other slots from the start
-        if (rec_cap == 0) {
-            int dev = 0, sms = 0;
-            if (cudaGetDevice(&dev) != cudaSuccess ||
-                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-                cudaGetLastError();
-                sms = 1;
-            }
-            rec_cap = std::max(1, sms * PGB_REC_BLOCKS_PER_SM);
-        }
-        const long long need = nrec > 0 ? ceil_div((long long)gn * nrec * rec_lanes, bz) : 0;
-        p.rec.blocks = (int)(dim == 2 ? std::min<long long>(need, (long long)rec_cap) : need);
     }
 
     void enqueue_forward(void* traces_out, cudaStream_t s) {
-        reset_task_counter(s);
         const size_t tr_group = (size_t)nsteps * nrec * sizeof(T);
         for (int g0 = 0; g0 < nshots; g0 += G) {
             int gn = std::min(G, nshots - g0);
@@ -1519,7 +1438,6 @@ struct PlanT final : public pysit_plan {
 
     void enqueue_gradient(const void* dobs, double* grad, double* rnorm2, void* traces_out, bool with_grad,
                           bool migrate, cudaStream_t s) {
-        reset_task_counter(s);
         const size_t tr_group = (size_t)nsteps * nrec * sizeof(T);
         if (with_grad) cudaMemsetAsync(ws + off.gpad, 0, (size_t)nx * ny * nz * sizeof(double), s);
         cudaMemsetAsync(ws + off.rnorm, 0, sizeof(double), s);
@@ -1651,7 +1569,7 @@ __global__ void lanes_sum_kernel(const double* __restrict__ g, int lanes, long l
 }
 
 // A plan whose shots are split into `lanes` contiguous ranges, each a plan of its own
-// (own workspace slice, streams and task counters), whose launch sequences run side by side:
+// (own workspace slice and streams), whose launch sequences run side by side:
 // forked from the caller's stream, joined back, captured in one graph.  The sequences never
 // wait for each other, so one lane's step kernels fill the gaps at the other's step
 // boundaries.  Gradients, images and misfits of the lanes are summed in a fixed order.

@@ -19,7 +19,7 @@ constexpr int kOZ = 4;    // z offset of cell k = 0 inside a row
 constexpr int kTailZ = 12;  // zero cells kept after the last cell of a row (>= halo + vector - 1)
 
 // bits of the device error word of a plan
-#define PGB_ERR_TIMEOUT 1    // a bounded wait for a bulk copy expired
+#define PGB_ERR_TIMEOUT 1    // a bounded device wait expired
 #define PGB_ERR_NONFINITE 2  // a NaN / Inf wavefield value (unstable time step)
 
 template <typename T> struct V16;
@@ -100,7 +100,6 @@ struct Record {
     T* traces;               // trace sample k of shot 0 receiver 0
     long long tr_sstride;    // stride between shots in the trace array
     int nrec;
-    int blocks;              // number of recorder blocks appended to the grid
     int lanes;               // threads per (shot, receiver): a power of two up to 32
 };
 
@@ -141,24 +140,14 @@ struct WaveParams {
     const T* m1;             // kBorn: edge-padded model perturbation (internal layout, shared by the shots);
                              // dw_in holds dWaveOp0_k
     int* err;                // device error word (PGB_ERR_* bits), may be NULL
-    unsigned polls;          // 0: a bulk-copy wait tries 2^22 times (each try may suspend); n: n non-blocking tests
-    int wait_fault;          // test aid: each task first waits (bounded) on a barrier nothing arrives on
+    unsigned polls;          // tests of the wait that wait_fault adds (0: 64)
+    int wait_fault;          // test aid: each 2D block first waits (bounded) on a barrier nothing arrives on
+    int pf_next;             // 2D: blocks fetch the next shot's tile into L2
     int psi_c2;              // 3D: 1 = C^2 multiplies sigma_x sigma_y sigma_z psi (the reference), 0 = not
     int nan_check;           // kRecomp: flag non-finite u_{k+1} as kFwd does (a forward sweep that keeps dWaveOp)
-    // 2D persistent sweep: task counters (interior, PML shell) shared by the
-    // launches of one run; this launch's tasks of kind 0 are the counter values
-    // task_base .. task_base + tasks - 1 of task_ctr[0], those of kind 1 start at
-    // task_base2 on task_ctr[1]
-    unsigned long long* task_ctr;
-    unsigned long long task_base, task_base2;
 };
 
 // ---- helpers shared by the 2D kernels ---------------------------------------
-template <typename T>
-__device__ __forceinline__ long long foff2(const WaveParams<T>& p, int x, int z) {
-    return (long long)(x + kHalo) * p.ldz + kOZ + z;
-}
-
 // rhs of one cell from the injection operator of its shot
 template <typename T>
 __device__ __forceinline__ T inject_rhs(const Inject<T>& inj, const int* bx, int shot, int x, int z) {
@@ -185,62 +174,70 @@ __device__ __forceinline__ T inject_rhs(const Inject<T>& inj, const int* bx, int
     return acc;
 }
 
-// trace recorder block: p.rec.lanes threads per (shot, receiver), the p.rec.blocks
-// recorder blocks striding over the receivers.  Lane l sums taps l, l + lanes, ... in
-// order, up to 8 of them with their loads in flight together; a fixed butterfly over the
-// lanes adds the partial sums, so the result does not depend on scheduling.  Every thread
-// of the block takes part (the butterfly shuffles over whole warps).
+// Trace recorder: p.rec.lanes threads per (shot, receiver), 32 / lanes receivers per warp pass.
+// Lane l sums taps l, l + lanes, ... in order, up to 8 of them with their loads in flight
+// together; a fixed butterfly over the lanes adds the partial sums, so the result does not
+// depend on scheduling.  Every lane of the warp takes part (the butterfly shuffles over it).
 template <typename T>
-__device__ __forceinline__ void record_block(const WaveParams<T>& p, int rb) {
+__device__ __forceinline__ long long record_passes(const WaveParams<T>& p) {
+    const int per = 32 / p.rec.lanes;
+    return p.rec.traces ? ((long long)p.nshot * p.rec.nrec + per - 1) / per : 0;
+}
+template <typename T>
+__device__ __forceinline__ void record_pass(const WaveParams<T>& p, long long pass) {
     constexpr int kTaps = 8;
     const int G = p.rec.lanes;
-    const long long t = (long long)rb * blockDim.x + threadIdx.x;
-    const int l = (int)(t & (G - 1));
-    const long long total = (long long)p.nshot * p.rec.nrec;
-    const long long pass = (long long)p.rec.blocks * blockDim.x / G;  // receivers per pass
-    for (long long base = 0; base < total; base += pass) {           // the same count on every lane
-        const long long id = base + t / G;
-        T acc = T(0);
-        if (id < total) {
-            const int shot = (int)(id / p.rec.nrec);
-            const int e1 = __ldg(p.rec.rowptr + id + 1);
-            const T* u = p.u_cur + (long long)shot * p.fstride;
-            for (int e = __ldg(p.rec.rowptr + id) + l; e < e1; e += kTaps * G) {
-                long long off[kTaps];
-                T w[kTaps], v[kTaps];
+    const int lane = threadIdx.x & 31, l = lane & (G - 1);
+    const long long id = pass * (32 / G) + lane / G;
+    const bool mine = id < (long long)p.nshot * p.rec.nrec;
+    int shot = 0;
+    T acc = T(0);
+    if (mine) {
+        shot = (int)(id / p.rec.nrec);
+        const int e1 = __ldg(p.rec.rowptr + id + 1);
+        const T* u = p.u_cur + (long long)shot * p.fstride;
+        for (int e = __ldg(p.rec.rowptr + id) + l; e < e1; e += kTaps * G) {
+            long long off[kTaps];
+            T w[kTaps], v[kTaps];
 #pragma unroll
-                for (int q = 0; q < kTaps; ++q) {
-                    const bool in = e + q * G < e1;
-                    off[q] = in ? __ldg(p.rec.off + e + q * G) : 0;
-                    w[q] = in ? __ldg(p.rec.w + e + q * G) : T(0);
-                }
-#pragma unroll
-                for (int q = 0; q < kTaps; ++q) v[q] = e + q * G < e1 ? __ldg(u + off[q]) : T(0);
-#pragma unroll
-                for (int q = 0; q < kTaps; ++q)
-                    if (e + q * G < e1) acc += w[q] * v[q];
+            for (int q = 0; q < kTaps; ++q) {
+                const bool in = e + q * G < e1;
+                off[q] = in ? __ldg(p.rec.off + e + q * G) : 0;
+                w[q] = in ? __ldg(p.rec.w + e + q * G) : T(0);
             }
-        }
-        for (int m = G >> 1; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
-        if (id < total && l == 0) {
-            const int shot = (int)(id / p.rec.nrec), r = (int)(id - (long long)shot * p.rec.nrec);
-            p.rec.traces[shot * p.rec.tr_sstride + r] = acc;
+#pragma unroll
+            for (int q = 0; q < kTaps; ++q) v[q] = e + q * G < e1 ? __ldg(u + off[q]) : T(0);
+#pragma unroll
+            for (int q = 0; q < kTaps; ++q)
+                if (e + q * G < e1) acc += w[q] * v[q];
         }
     }
+    for (int m = G >> 1; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
+    if (mine && l == 0) p.rec.traces[shot * p.rec.tr_sstride + (id - (long long)shot * p.rec.nrec)] = acc;
 }
 
-// persistent-warp 2D sweep fed by shared-memory row rings, one task kind per
-// kernel (0 interior, 1 PML shell); tasks = [ntasks][5] ints (x0, x1, zs, ze,
-// kind) of one shot, shared by all shots; `blocks` task blocks.  Returns the
-// number of task-counter values the launch consumes.
-template <typename T, int R, int MODE, int KIND>
-long long launch_wave2d_warp_tasks(const WaveParams<T>& p, const int* tasks, int ntasks, int blocks,
-                                   cudaStream_t s);
-int wave2d_warp_threads();
-int wave2d_warp_seg(int dtype_bytes, int order, int pml);
-// resident task blocks of the whole GPU for one (dtype, order, mode, kind)
-int wave2d_warp_blocks(int dtype_bytes, int order, int mode, int kind);
-void wave2d_warp_prepare();
+// 2D tiles of one shot, shared by all shots: the device's form of the task table, interior
+// tiles first
+struct Tile2d {
+    int x0, rows, zs, ncell;    // rows x0 .. x0+rows-1, cells zs .. zs+ncell-1
+    int nzv, inv, kind, pad;    // vectors along z, ceil(2^16 / nzv), 0 interior / 1 PML shell
+};
+constexpr int kT2 = 128;  // threads of a block
+// `strip`: x-rows per thread (1, 2 or 4); `inj_cap`: cells of the largest tile's part of any
+// shot's injection box
+template <typename T, int R, int MODE>
+void launch_wave2d_tiles(const WaveParams<T>& p, const Tile2d* tiles, int nint, int nshell, int strip, int inj_cap,
+                         cudaStream_t s);
+// cells of a thread along z: a 16-byte vector; an FP32 shell thread takes two cells (its two
+// column and two window sets of registers are twice the interior's)
+constexpr int wave2d_cells(int dtype_bytes, int pml) { return dtype_bytes == 4 && !pml ? 4 : 2; }
+// widest z-range of a tile of each kind: 32 threads
+constexpr int wave2d_seg(int dtype_bytes, int pml) { return 32 * wave2d_cells(dtype_bytes, pml); }
+// x-rows a block's threads take side by side, `strip` rows each
+constexpr int wave2d_tile_rows(int dtype_bytes, int pml, int strip, int zcells) {
+    const int V = wave2d_cells(dtype_bytes, pml);
+    return kT2 / ((zcells + V - 1) / V) * strip;
+}
 // 3D block tasks (x0, x1, y0, y1, zs, ze): one block per task and shot (KIND 0
 // interior, 1 PML shell); a warp takes 32 / (vectors of the z-range) y-rows
 template <typename T, int R, int MODE, int KIND>

@@ -1,0 +1,6 @@
+// 2D tile kernels, double, order 6 (one translation unit per type and order: they compile side by side)
+#include "wave2d_tile.cuh"
+
+namespace pgb {
+PGB_INSTANTIATE_2D(double, 3)
+}  // namespace pgb

@@ -136,10 +136,9 @@ class WavePlan:
         ``forward_only`` plans model data only (no adjoint, imaging or checkpoint storage).
         ``lanes`` (default 1): the shots split into that many ranges whose launch sequences run
         side by side on their own streams, shots_per_launch being per lane.
-        ``wait_polls`` (default 0, the library's limit): tries of a step kernel's wait for a
-        bulk copy before it counts as expired (``check_status`` then raises).  ``wait_fault``
-        (test aid): the 2D step kernels' tasks first wait on a barrier nothing arrives on, so
-        that the wait runs out and the expiry path runs."""
+        ``wait_fault`` (test aid): the 2D step kernels' blocks first wait on a barrier nothing
+        arrives on, so that the wait runs out (``check_status`` then raises); ``wait_polls``:
+        tests of that wait (0: the library's default)."""
         torch = _native.require_cuda()
         lib = _native.load()
         self.solver = solver
@@ -487,20 +486,20 @@ class WavePlan:
                                                            C.c_void_p(_native.stream_handle())))
 
     def status(self):
-        """Device status flags (1: bulk-copy wait expired, 2: non-finite wavefield); clears them."""
+        """Device status flags (1: a device wait expired, 2: non-finite wavefield); clears them."""
         f = C.c_int()
         _native.check(_native.load().pysit_plan_status(self._h, C.byref(f), C.c_void_p(_native.stream_handle())))
         return int(f.value)
 
     def check_status(self):
         """Read and clear the status flags of the runs since the last read.  An expired
-        bulk-copy wait (flag 1) makes those runs' results invalid: PysitCudaError with
+        device wait (flag 1) makes those runs' results invalid: PysitCudaError with
         PYSIT_ETIMEOUT.  A non-finite wavefield (flag 2: the time step is unstable) is left to
         the caller, as the reference leaves it: the flags are returned."""
         f = self.status()
         if f & 1:
             raise _native.PysitCudaError(
-                _native.PYSIT_ETIMEOUT, "a step kernel's wait for a bulk copy expired: the results of the "
+                _native.PYSIT_ETIMEOUT, "a step kernel's device wait expired: the results of the "
                 "plan's last runs are invalid")
         return f
 
