@@ -107,7 +107,7 @@ __global__ void inject_scatter3d_kernel(const WaveParams<T> p, int cells_max) {
 // Born source of one step added after the stencil kernels of the scattered field u1:
 //     u1_{k+1} += fac C^2 rhs1,   rhs1 = -m1 dWaveOp0_k
 // (TemporalModeling.linear_forward_model, pysit/modeling/temporal_modeling.py:520-525; the
-// step is linear in rhs, fac as in inject_scatter3d_kernel).  One block per row
+// step is linear in rhs, fac as in the 3D kernel's inject_fac).  One block per row
 // (shot, x, y) of the padded grid, threads along z; cells of the outer ring are skipped as
 // the reference's step skips them.  m1 and C^2 are shared by the shots; dw holds dWaveOp0_k
 // of every shot of the launch.
@@ -149,14 +149,6 @@ __global__ void edge_pad_kernel(const double* __restrict__ m, int nx, int ny, in
         const int ii = min(max(i - lx, 0), px - 1), jj = min(max(j - ly, 0), py - 1), kk = min(max(k - lz, 0), pz - 1);
         out[ioff(i, j, k, hx, hy, rows_y, ldz)] = T(m[((long long)ii * py + jj) * pz + kk]);
     }
-}
-
-// trace recorder as a kernel of its own (runs beside the stencil kernels: it only reads u_k)
-constexpr int kRecThreads = 128;
-template <typename T>
-__global__ void __launch_bounds__(kRecThreads) record_kernel(const WaveParams<T> p) {
-    const long long pass = (long long)blockIdx.x * (kRecThreads / 32) + (threadIdx.x >> 5);
-    if (pass < record_passes(p)) record_pass(p, pass);
 }
 
 constexpr int kRedBlocks = 1024;
@@ -325,17 +317,17 @@ struct PlanT final : public pysit_plan {
     int nseg;
     std::vector<int> tasks2d;    // [ntasks][5] tiles of the 2D step: interior first, then shell
     int ntask2d[2] = {0, 0};     // tasks of each kind
-    std::vector<int> tasks3d;    // [ntasks][6] block tasks of the 3D sweep: interior first, then shell
+    std::vector<int> tasks3d;    // [ntasks][6] tiles of the 3D step: interior first, then shell
+    std::vector<Tile3d> tiles3d; // 3D: the device's form of tasks3d
     int ntask3d[2] = {0, 0};
+    int planes3d = 4;            // 3D: x-planes per thread and round
     int strip2d = 4;             // 2D: x-rows per thread of a tile
     std::vector<Tile2d> tiles2d;      // 2D: the device's form of tasks2d
-    int inj_cap[2] = {0, 0};     // 2D: injection cells of a tile at most (source, receivers)
+    int inj_cap[2] = {0, 0};     // 2D, 3D: injection cells of a tile at most (source, receivers)
     double shell_frac[4] = {0.0, 0.0, 0.0, 0.0};  // descriptor's shell shares (read back by tuning(); unused)
-    cudaStream_t aux = nullptr;  // second stream of the 3D step (shell kernel beside the interior one)
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     // ---- acquisition (host) ----------------------------------------------------
     std::vector<CSRBox> src_inj, rec_inj;
-    int rec_box_max = 0;              // largest receiver injection box (cells) over the shots
+    int rec_box_max = 0;              // 3D: largest receiver injection box (cells) over the shots
     std::vector<int> rec_rows;        // [nshots*nrec+1]
     int rec_lanes = 1;                // recorder threads per (shot, receiver)
     std::vector<long long> rec_off;   // internal offsets
@@ -382,9 +374,6 @@ struct PlanT final : public pysit_plan {
         for (auto& kv : graphs)
             if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
         if (cap) cudaStreamDestroy(cap);
-        if (aux) cudaStreamDestroy(aux);
-        if (ev_fork) cudaEventDestroy(ev_fork);
-        if (ev_join) cudaEventDestroy(ev_join);
     }
 
     template <typename U>
@@ -465,6 +454,7 @@ struct PlanT final : public pysit_plan {
         for (auto& b : rec_inj)
             rec_box_max = std::max(rec_box_max, (b.box[1] - b.box[0]) * (b.box[3] - b.box[2]) * (b.box[5] - b.box[4]));
         if (dim == 2) size_tiles2d();
+        if (dim == 3) build_tasks3d();  // sized by the injection boxes
         rc = build_recording(d);
         if (rc) return rc;
         src_amp.assign(d.src_amp, d.src_amp + (size_t)nshots * nsteps * nsrc);
@@ -483,8 +473,7 @@ struct PlanT final : public pysit_plan {
             return;
         }
         if (dim == 3) {
-            bz = 128;  // threads of the recorder blocks
-            tx = tile_req ? tile_req : 64;
+            choose_tile3d();
             build_tasks3d();
             ntz = ntx = 1;
             return;
@@ -609,28 +598,73 @@ struct PlanT final : public pysit_plan {
         add_tasks(xa, xb, zb, nz, 1);   // high-z band
     }
 
-    // 3D block tasks: the interior box (R cells clear of the padding, off the outer
-    // ring, z-bounds multiples of 4) and the six slabs of the shell around it; x in
+    // Planes per thread and round, and the default task length, of the 3D tiles: four planes share
+    // the most loads, and longer tiles the planes that successive rounds meet in L1, but both make
+    // fewer blocks; a launch keeps about four waves of the GPU's 304 resident blocks.  Measured
+    // (us per forward step, planes x length): 440 x 440 x 340 order 8 FP32 4x32 515 (adjoint 709),
+    // 4x16 520 (691), 4x8 535 (684), 4x64 542 (750), 1x8 616; 121 x 107 x 95 order 4 FP32 x 4 shots 4x4 101, 4x8 103, 4x16 122, 1x4 106;
+    // 53 x 49 x 45 order 4 FP64 x 2 shots 1x1 72, 1x4 91, 4x4 86, 4x16 133
+    void choose_tile3d() {
+        const long long blocks = (long long)nx * ny * nz * G / (kT3 * (16 / (int)sizeof(T)));  // of one plane each
+        planes3d = blocks >= 4 * 304 ? 4 : 1;
+        tx = 1;
+        if (planes3d > 1)
+            for (tx = 4; tx < 16 && blocks / (2 * tx) >= 4 * 304; tx *= 2) {}
+        if (tile_req) tx = tile_req;
+    }
+
+    // 3D tiles: the interior box (R cells clear of the padding, off the outer
+    // ring, z-bounds multiples of 4) and the shell around it: six slabs, each cut into the part
+    // where its own axis alone may be in the padding (a face) and the rest; x in
     // chunks of about tx rows, z in segments, y in groups of the rows one block
-    // covers (a shell warp takes several rows of a narrow z segment).
-    // Consecutive tasks are neighbouring y-groups (their halo rows meet in L2).
+    // covers (a warp takes several rows of a narrow z segment).
+    // Consecutive tiles are neighbouring y-groups (their halo rows meet in L2).
     void add_tasks3d(int xa, int xb, int ya, int yb, int za, int zb, int kind) {
         if (xb <= xa || yb <= ya || zb <= za) return;
+        constexpr int V = V16<T>::N;
         std::vector<std::pair<int, int>> zs;
-        int w = wave3d_seg((int)sizeof(T), kind);
+        int w = wave3d_seg((int)sizeof(T));
         if (kind == 0 && tz > 0) w = std::min(w, tz);
         split3d(za, zb, w, zs);
         const int nxc = (xb - xa + tx - 1) / tx, wx = (xb - xa + nxc - 1) / nxc;
         for (int x = xa; x < xb; x += wx)
-            for (auto& z : zs)
-                for (int y = ya, rows = wave3d_task_rows((int)sizeof(T), kind, z.second - z.first); y < yb;
-                     y += rows) {
+            for (auto& z : zs) {
+                const int nzv = (z.second - z.first + V - 1) / V;
+                for (int y = ya, rows = wave3d_task_rows((int)sizeof(T), z.second - z.first); y < yb; y += rows) {
                     int t[6] = {x, std::min(xb, x + wx), y, std::min(yb, y + rows), z.first, z.second};
                     tasks3d.insert(tasks3d.end(), t, t + 6);
+                    tiles3d.push_back({t[0], t[1], t[2], t[3], t[4], t[5], kind, (65536 + nzv - 1) / nzv});
                 }
+            }
+    }
+    // the injection boxes' largest part in a tile; false when it does not fit the kernel's buffer
+    bool size_tiles3d() {
+        auto cells = [&](const std::vector<CSRBox>& v) {
+            long long most = 0;
+            for (auto& b : v)
+                for (auto& t : tiles3d) {
+                    const long long dx = std::min(b.box[1], t.x1) - std::max(b.box[0], t.x0);
+                    const long long dy = std::min(b.box[3], t.y1) - std::max(b.box[2], t.y0);
+                    const long long dz = std::min(b.box[5], t.ze) - std::max(b.box[4], t.zs);
+                    if (dx > 0 && dy > 0 && dz > 0) most = std::max(most, dx * dy * dz);
+                }
+            return (int)((most + 3) / 4 * 4);
+        };
+        inj_cap[0] = cells(src_inj);
+        inj_cap[1] = cells(rec_inj);
+        return inj_cap[0] * sizeof(T) <= (size_t)kMaxInj3d;  // (receivers: at most 4 kT3 cells, or scattered)
     }
     void build_tasks3d() {
+        const int keep = tx;
+        for (;; tx = std::max(1, tx / 2)) {  // shorter tiles until every tile's injection fits
+            build_tasks3d_();
+            if (size_tiles3d() || tx == 1) break;
+        }
+        tx = keep;
+    }
+    void build_tasks3d_() {
         tasks3d.clear();
+        tiles3d.clear();
         const int xa = pl[0] > 0 ? pl[0] + R : 1, xb = pr[0] > 0 ? nx - pr[0] - R : nx - 1;
         const int ya = pl[1] > 0 ? pl[1] + R : 1, yb = pr[1] > 0 ? ny - pr[1] - R : ny - 1;
         const int za = ((pl[2] > 0 ? pl[2] + R : 1) + 3) / 4 * 4;
@@ -640,15 +674,27 @@ struct PlanT final : public pysit_plan {
             add_tasks3d(0, nx, 0, ny, 0, nz, 1);
         } else {
             add_tasks3d(xa, xb, ya, yb, za, zb, 0);
-            ntask3d[0] = (int)(tasks3d.size() / 6);
-            add_tasks3d(0, xa, 0, ny, 0, nz, 1);    // low-x slab
-            add_tasks3d(xb, nx, 0, ny, 0, nz, 1);   // high-x slab
-            add_tasks3d(xa, xb, 0, ya, 0, nz, 1);   // low-y slab
-            add_tasks3d(xa, xb, yb, ny, 0, nz, 1);  // high-y slab
-            add_tasks3d(xa, xb, ya, yb, 0, za, 1);  // low-z slab
-            add_tasks3d(xa, xb, ya, yb, zb, nz, 1); // high-z slab
+            ntask3d[0] = (int)tiles3d.size();
+            // off the padding: y in [y0, y1); z in [z0, z1) (multiples of 4, or the grid's end)
+            const int y0 = pl[1], y1 = ny - pr[1];
+            const int z0 = (pl[2] + 3) / 4 * 4, z1 = pr[2] > 0 ? (nz - pr[2]) / 4 * 4 : nz;
+            // edges and corners first (the longest tiles), then the faces
+            for (int side = 0; side < 2; ++side) {
+                const int x0 = side ? xb : 0, x1 = side ? nx : xa;
+                add_tasks3d(x0, x1, 0, y0, 0, nz, 1);
+                add_tasks3d(x0, x1, y1, ny, 0, nz, 1);
+                add_tasks3d(x0, x1, y0, y1, 0, z0, 1);
+                add_tasks3d(x0, x1, y0, y1, z1, nz, 1);
+                add_tasks3d(xa, xb, side ? yb : 0, side ? ny : ya, 0, z0, 1);
+                add_tasks3d(xa, xb, side ? yb : 0, side ? ny : ya, z1, nz, 1);
+            }
+            for (int side = 0; side < 2; ++side) {
+                add_tasks3d(side ? xb : 0, side ? nx : xa, y0, y1, z0, z1, 2);
+                add_tasks3d(xa, xb, side ? yb : 0, side ? ny : ya, z0, z1, 3);
+                add_tasks3d(xa, xb, ya, yb, side ? zb : 0, side ? nz : za, 4);
+            }
         }
-        ntask3d[1] = (int)(tasks3d.size() / 6) - ntask3d[0];
+        ntask3d[1] = (int)tiles3d.size() - ntask3d[0];
     }
 
     // ints of the task table for a task length tx_try and z extent tz_try (the current table is kept)
@@ -802,7 +848,7 @@ struct PlanT final : public pysit_plan {
         // not always enough to make up for the extra segments)
         task_cap = std::max<size_t>(task_ints(kMinTileX, 0), std::max(tasks2d.size(), tasks3d.size()));
         for (int z = kMinTileZ; z <= 32 * V16<T>::N; z += 4) task_cap = std::max(task_cap, task_ints(kMinTileX, z));
-        off.tasks = take(std::max<size_t>(dim == 2 ? task_cap / 5 * sizeof(Tile2d) : task_cap * sizeof(int), sizeof(Tile2d)));
+        off.tasks = take(std::max<size_t>(dim == 2 ? task_cap / 5 * sizeof(Tile2d) : task_cap / 6 * sizeof(Tile3d), sizeof(Tile3d)));
         off.partial = take(kRedBlocks * sizeof(double));
         off.rnorm = take(sizeof(double));
         ws_need = tot;
@@ -865,14 +911,15 @@ struct PlanT final : public pysit_plan {
         if ((rc = upload_inj(rec_inj, off.rbox, off.rrpb, off.rrow, off.rpt, off.rw, s))) return rc;
         if ((rc = upload(off.recrow, rec_rows, s)) || (rc = upload(off.recoff, rec_off, s))) return rc;
         if ((rc = upload(off.recw, tmp = toT(rec_ws), s))) return rc;
-        if ((rc = dim == 3 ? upload(off.tasks, tasks3d, s) : upload(off.tasks, tiles2d, s))) return rc;
+        if ((rc = dim == 3 ? upload(off.tasks, tiles3d, s) : upload(off.tasks, tiles2d, s))) return rc;
         if ((rc = upload(off.shsteps, shot_steps, s))) return rc;
         PGB_CHECK_CUDA(cudaStreamSynchronize(s));
         if (!cap) PGB_CHECK_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
-        if (dim == 3) {
-            if (!aux) PGB_CHECK_CUDA(cudaStreamCreateWithFlags(&aux, cudaStreamNonBlocking));
-            if (!ev_fork) PGB_CHECK_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
-            if (!ev_join) PGB_CHECK_CUDA(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
+        if (dim == 3) switch (R) {
+            case 1: wave3d_tile_prepare<T, 1>(); break;
+            case 2: wave3d_tile_prepare<T, 2>(); break;
+            case 3: wave3d_tile_prepare<T, 3>(); break;
+            default: wave3d_tile_prepare<T, 4>(); break;
         }
         PGB_CHECK_CUDA(cudaGetLastError());
         model_set = false;
@@ -962,39 +1009,18 @@ struct PlanT final : public pysit_plan {
         ++launches;
     }
 
-    // One 3D step: interior kernel on s, PML-shell kernel (and the trace recorder)
-    // on the auxiliary stream, forked and joined as in 2D; the adjoint source is
-    // added after the step by a scatter kernel.
+    // One 3D step: as in 2D, one launch over the tiles of every shot.  An adjoint source of more
+    // than a few cells per thread of a tile (long tiles under a dense receiver patch) would hold
+    // the tile's block back (z-face tiles of the 440 x 440 x 340 grid with 100 x 100 receivers, 5120
+    // cells a tile: 248 against 185 us) and is added by a scatter kernel after the step.
     template <int RR, int MODE>
     void launch3d(const WaveParams<T>& p, cudaStream_t s) {
-        const int* tk = at<int>(off.tasks);
         WaveParams<T> q = p;
-        const bool scatter = MODE == kAdj && q.inj.on && rec_box_max > 0;
+        const bool scatter = MODE == kAdj && q.inj.on && inj_cap[1] > 4 * kT3;
         if (scatter) q.inj.on = 0;
-        const bool rec = MODE != kAdj && q.rec.traces && q.rec.nrec > 0;
-        const bool fork = ntask3d[0] > 0 && (ntask3d[1] > 0 || rec);
-        cudaStream_t side = fork ? aux : s;
-        if (fork) {
-            cudaEventRecord(ev_fork, s);
-            cudaStreamWaitEvent(aux, ev_fork, 0);
-        }
-        if (rec) {
-            const long long passes = ((long long)q.nshot * q.rec.nrec * q.rec.lanes + 31) / 32;
-            record_kernel<T><<<(int)((passes * 32 + kRecThreads - 1) / kRecThreads), kRecThreads, 0, side>>>(q);
-            ++launches;
-        }
-        if (ntask3d[1] > 0) {
-            launch_wave3d_tasks<T, RR, MODE, 1>(q, tk + 6 * ntask3d[0], ntask3d[1], side);
-            ++launches;
-        }
-        if (ntask3d[0] > 0) {
-            launch_wave3d_tasks<T, RR, MODE, 0>(q, tk, ntask3d[0], s);
-            ++launches;
-        }
-        if (fork) {
-            cudaEventRecord(ev_join, aux);
-            cudaStreamWaitEvent(s, ev_join, 0);
-        }
+        launch_wave3d_tiles<T, RR, MODE>(q, at<Tile3d>(off.tasks), ntask3d[0], ntask3d[1], planes3d,
+                                         scatter ? 0 : inj_cap[MODE == kAdj], s);
+        ++launches;
         if (scatter) {
             q.inj.on = 1;
             const long long n = (long long)q.nshot * rec_box_max;
@@ -1405,7 +1431,7 @@ struct PlanT final : public pysit_plan {
         tz = z > 0 ? z / 4 * 4 : 0;
         std::vector<int>& tab = dim == 3 ? (build_tasks3d(), tasks3d) : (build_tasks2d(), tasks2d);
         PGB_REQUIRE(tab.size() <= task_cap, "task table of %zu ints exceeds its buffer (%zu)", tab.size(), task_cap);
-        int rc = dim == 3 ? upload(off.tasks, tasks3d, s) : upload(off.tasks, tiles2d, s);
+        int rc = dim == 3 ? upload(off.tasks, tiles3d, s) : upload(off.tasks, tiles2d, s);
         if (rc) return rc;
         PGB_CHECK_CUDA(cudaStreamSynchronize(s));
         for (auto& kv : graphs)

@@ -174,6 +174,19 @@ __device__ __forceinline__ T inject_rhs(const Inject<T>& inj, const int* bx, int
     return acc;
 }
 
+template <typename T>
+__device__ __forceinline__ T inject_rhs3(const Inject<T>& inj, const int* bx, int shot, int x,
+                                         int y, int z) {
+    if (x < bx[0] || x >= bx[1] || y < bx[2] || y >= bx[3] || z < bx[4] || z >= bx[5]) return T(0);
+    long long c = ((long long)(x - bx[0]) * (bx[3] - bx[2]) + (y - bx[2])) * (bx[5] - bx[4]) + (z - bx[4]);
+    const int* rp = inj.rowptr + inj.rpbase[shot];
+    int e0 = __ldg(rp + c), e1 = __ldg(rp + c + 1);
+    const T* amp = inj.amp + shot * inj.amp_sstride;
+    T acc = T(0);
+    for (int e = e0; e < e1; ++e) acc += __ldg(inj.w + e) * __ldg(amp + __ldg(inj.pt + e));
+    return acc;
+}
+
 // Trace recorder: p.rec.lanes threads per (shot, receiver), 32 / lanes receivers per warp pass.
 // Lane l sums taps l, l + lanes, ... in order, up to 8 of them with their loads in flight
 // together; a fixed butterfly over the lanes adds the partial sums, so the result does not
@@ -238,12 +251,28 @@ constexpr int wave2d_tile_rows(int dtype_bytes, int pml, int strip, int zcells) 
     const int V = wave2d_cells(dtype_bytes, pml);
     return kT2 / ((zcells + V - 1) / V) * strip;
 }
-// 3D block tasks (x0, x1, y0, y1, zs, ze): one block per task and shot (KIND 0
-// interior, 1 PML shell); a warp takes 32 / (vectors of the z-range) y-rows
-template <typename T, int R, int MODE, int KIND>
-void launch_wave3d_tasks(const WaveParams<T>& p, const int* tasks, int ntasks, cudaStream_t s);
-int wave3d_seg(int dtype_bytes, int kind);  // widest z-range of a task of each kind
-int wave3d_task_rows(int dtype_bytes, int kind, int zcells);  // y-rows of a task of zcells z-cells
+// 3D tiles of one shot, shared by all shots: the device's form of the task table, interior
+// tiles first
+struct Tile3d {
+    int x0, x1, y0, y1;     // planes and rows
+    int zs, ze, kind, inv;  // cells along z; 0 interior, 1 general shell, 2-4 faces; ceil(2^16 / vectors along z)
+};
+constexpr int kT3 = 256;                 // threads of a block
+constexpr int kMaxInj3d = 160 * 1024;    // bytes of injection cells of a tile at most
+// `planes`: x-planes per thread and round (1 or 4); `inj_cap`: cells of the largest tile's part of
+// any shot's injection box
+template <typename T, int R, int MODE>
+void launch_wave3d_tiles(const WaveParams<T>& p, const Tile3d* tiles, int nint, int nshell, int planes, int inj_cap,
+                         cudaStream_t s);
+template <typename T, int R>
+void wave3d_tile_prepare();
+// widest z-range of a tile: 32 vectors
+constexpr int wave3d_seg(int dtype_bytes) { return 32 * (16 / dtype_bytes); }
+// y-rows of a tile of zcells z-cells: a warp takes 32 / vectors rows
+constexpr int wave3d_task_rows(int dtype_bytes, int zcells) {
+    const int V = 16 / dtype_bytes;
+    return kT3 / 32 * (32 / ((zcells + V - 1) / V));
+}
 template <typename T, int R, int MODE>
 void launch_wave1d(const WaveParams<T>& p, int bz, cudaStream_t s);
 

@@ -39,139 +39,11 @@
 // shots forward 159-178 us with four single-stage blocks per SM, 255-350 us with persistent
 // blocks, two stages and a copying warp).
 #pragma once
+#include "pairs.cuh"
 #include "tma.cuh"
-#include "wave.cuh"
 
 namespace pgb {
 namespace {
-
-// Pair arithmetic: two neighbouring cells per operation.  FP32 uses the packed f32x2
-// instructions on 64-bit registers (one issue slot for two cells, each half rounded exactly
-// like the scalar operation; the pairs stay packed from load to store, since taking them
-// apart costs as many moves as the arithmetic saves); FP64 spells the pair out.
-template <typename T> struct PairOps;
-template <> struct PairOps<float> {
-    using P = unsigned long long;
-    static __device__ __forceinline__ P mk(float a, float b) {
-        P d;
-        asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
-        return d;
-    }
-    static __device__ __forceinline__ float lo(P a) { return __uint_as_float((unsigned)a); }
-    static __device__ __forceinline__ float hi(P a) { return __uint_as_float((unsigned)(a >> 32)); }
-    static __device__ __forceinline__ P dup(float a) { return mk(a, a); }
-    static __device__ __forceinline__ P add(P a, P b) {
-        P d;
-        asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-        return d;
-    }
-    static __device__ __forceinline__ P sub(P a, P b) {
-        P d;
-        asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-        return d;
-    }
-    static __device__ __forceinline__ P mul(P a, P b) {
-        P d;
-        asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-        return d;
-    }
-    static __device__ __forceinline__ P fma(P a, P b, P c) {
-        P d;
-        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-        return d;
-    }
-};
-template <> struct PairOps<double> {
-    using P = double2;
-    static __device__ __forceinline__ P mk(double a, double b) { return make_double2(a, b); }
-    static __device__ __forceinline__ double lo(P a) { return a.x; }
-    static __device__ __forceinline__ double hi(P a) { return a.y; }
-    static __device__ __forceinline__ P dup(double a) { return make_double2(a, a); }
-    static __device__ __forceinline__ P add(P a, P b) { return make_double2(a.x + b.x, a.y + b.y); }
-    static __device__ __forceinline__ P sub(P a, P b) { return make_double2(a.x - b.x, a.y - b.y); }
-    static __device__ __forceinline__ P mul(P a, P b) { return make_double2(a.x * b.x, a.y * b.y); }
-    static __device__ __forceinline__ P fma(P a, P b, P c) {
-        return make_double2(::fma(a.x, b.x, c.x), ::fma(a.y, b.y, c.y));
-    }
-};
-// N pairs of neighbouring cells: a thread's vector along z
-template <typename T, int N>
-struct Pairs {
-    typename PairOps<T>::P p[N];
-};
-__device__ __forceinline__ void ldp(Pairs<float, 2>& r, const float* q) {
-    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(q);
-    r.p[0] = v.x; r.p[1] = v.y;
-}
-__device__ __forceinline__ void ldp(Pairs<float, 1>& r, const float* q) { r.p[0] = *reinterpret_cast<const unsigned long long*>(q); }
-__device__ __forceinline__ void ldp(Pairs<double, 1>& r, const double* q) { r.p[0] = *reinterpret_cast<const double2*>(q); }
-__device__ __forceinline__ void stp(float* q, const Pairs<float, 2>& r) { *reinterpret_cast<ulonglong2*>(q) = make_ulonglong2(r.p[0], r.p[1]); }
-__device__ __forceinline__ void stp(float* q, const Pairs<float, 1>& r) { *reinterpret_cast<unsigned long long*>(q) = r.p[0]; }
-__device__ __forceinline__ void stp(double* q, const Pairs<double, 1>& r) { *reinterpret_cast<double2*>(q) = r.p[0]; }
-__device__ __forceinline__ void stp_cs(float* q, const Pairs<float, 2>& r) { __stcs(reinterpret_cast<ulonglong2*>(q), make_ulonglong2(r.p[0], r.p[1])); }
-__device__ __forceinline__ void stp_cs(float* q, const Pairs<float, 1>& r) { __stcs(reinterpret_cast<unsigned long long*>(q), r.p[0]); }
-__device__ __forceinline__ void stp_cs(double* q, const Pairs<double, 1>& r) { __stcs(reinterpret_cast<double2*>(q), r.p[0]); }
-
-// a thread's cells of one row with NB vectors of NP pairs on either side.  Taps an odd number
-// of cells away straddle two pairs: in FP32 they are taken cell by cell (putting the pairs
-// together costs more moves than the packed operation saves).
-template <typename T, int NP, int NB>
-struct Window {
-    using O = PairOps<T>;
-    using P = typename O::P;
-    static constexpr int N = (2 * NB + 1) * NP;
-    P e[N];
-    __device__ __forceinline__ void load(const T* q, const Pairs<T, NP>* centre) {
-#pragma unroll
-        for (int j = 0; j <= 2 * NB; ++j) {
-            Pairs<T, NP> a;
-            if (j == NB && centre) a = *centre;
-            else ldp(a, q + j * 2 * NP);
-#pragma unroll
-            for (int k = 0; k < NP; ++k) e[j * NP + k] = a.p[k];
-        }
-    }
-    __device__ __forceinline__ T cell(int i) const { return i & 1 ? O::hi(e[i >> 1]) : O::lo(e[i >> 1]); }
-    // the pair of cells i, i + 1
-    __device__ __forceinline__ P at(int i) const { return i & 1 ? O::mk(cell(i), cell(i + 1)) : e[i >> 1]; }
-    // acc + wd ((v_{c+d} - v_c) + (v_{c-d} - v_c)) for the pair at cell c
-    __device__ __forceinline__ P d2(P acc, P wd, int c, int d) const {
-        if (d & 1) {
-            const P uc = e[c >> 1];
-            const T a = (cell(c + d) - O::lo(uc)) + (cell(c - d) - O::lo(uc));
-            const T b = (cell(c + 1 + d) - O::hi(uc)) + (cell(c + 1 - d) - O::hi(uc));
-            return O::mk(::fma(O::lo(wd), a, O::lo(acc)), ::fma(O::hi(wd), b, O::hi(acc)));
-        }
-        return O::fma(wd, O::add(O::sub(e[(c + d) >> 1], e[c >> 1]), O::sub(e[(c - d) >> 1], e[c >> 1])), acc);
-    }
-    // acc + wd (v_{c+d} - v_{c-d})
-    __device__ __forceinline__ P d1(P acc, P wd, int c, int d) const {
-        if (d & 1)
-            return O::mk(::fma(O::lo(wd), cell(c + d) - cell(c - d), O::lo(acc)),
-                         ::fma(O::hi(wd), cell(c + 1 + d) - cell(c + 1 - d), O::hi(acc)));
-        return O::fma(wd, O::sub(e[(c + d) >> 1], e[(c - d) >> 1]), acc);
-    }
-};
-
-// weights of the derivatives over the first differences e_j = v_{j+1} - v_j (FP64 path):
-// v'' = sum_j c_j (e_j - e_{-1-j}), v' = sum_j b_j (e_j + e_{-1-j}), j = 0..R-1, with
-// c_j = sum_{m>j} w2_m and b_j = sum_{m>j} w1_m
-__host__ __device__ constexpr double c2sum(int R, int j) {
-    double s = 0;
-    for (int m = j + 1; m <= R; ++m) s += d2w(R, m);
-    return s;
-}
-__host__ __device__ constexpr double c1sum(int R, int j) {
-    double s = 0;
-    for (int m = j + 1; m <= R; ++m) s += d1w(R, m);
-    return s;
-}
-
-template <typename T> __device__ __forceinline__ T rcp_(T x);
-// FP32: the fast reciprocal (within ~1 ulp; the FP32 path's tolerances are 1e-4 / 1e-3);
-// FP64 keeps the exact division of the reference
-template <> __device__ __forceinline__ float rcp_(float x) { return __fdividef(1.0f, x); }
-template <> __device__ __forceinline__ double rcp_(double x) { return 1.0 / x; }
 
 // One thread's strip of a tile: RS consecutive x-rows of one vector along z, operands read
 // straight from global memory (L1 serves the rows and vectors that neighbouring threads share).
@@ -221,17 +93,17 @@ __device__ __forceinline__ void tile_update(const WaveParams<T>& p, const T* rhs
     // rows past the tile's last one are read too (the next rows of the field, or its halo:
     // clamped to the strip's last row that exists) and not used
 #pragma unroll
-    for (int j = 0; j < RS + 2 * R; ++j) ldp(cv[j], u + (long long)(min(j, rows - r0 + 2 * R - 1) - R) * ldz);
+    for (int j = 0; j < RS + 2 * R; ++j) ldr(cv[j], u + (long long)(min(j, rows - r0 + 2 * R - 1) - R) * ldz);
 #pragma unroll
     for (int r = 0; r < RS; ++r) {
         const long long d = (long long)min(r, rows - r0 - 1) * ldz;
         ldp(um[r], p.u_prev + sh + o0 + d);
-        ldp(cc[r], p.c2 + o0 + d);
+        ldr(cc[r], p.c2 + o0 + d);
     }
     if (PML) {
 #pragma unroll
         for (int j = 0; j < RS + 2 * R; ++j)
-            ldp(px[j], p.phx_in + sh + o0 + (long long)(min(j, rows - r0 + 2 * R - 1) - R) * ldz);
+            ldr(px[j], p.phx_in + sh + o0 + (long long)(min(j, rows - r0 + 2 * R - 1) - R) * ldz);
     }
     {
 #pragma unroll
@@ -243,8 +115,8 @@ __device__ __forceinline__ void tile_update(const WaveParams<T>& p, const T* rhs
             w.load(u + (long long)r * ldz - HZ, &cv[R + r]);
             Pairs<T, NP> dwi, ici;
             if ((MODE == kAdj && img) || MODE == kBorn) {  // for kBorn: dWaveOp0 and m1
-                ldp(dwi, p.dw_in + sh + o);
-                if (MODE == kBorn) ldp(ici, p.m1 + o);
+                ldr(dwi, p.dw_in + sh + o);
+                if (MODE == kBorn) ldr(ici, p.m1 + o);
                 else ldp(ici, p.ic + sh + o);
             }
             T sx = T(0), mgx = T(0);

@@ -1,0 +1,6 @@
+// 3D tile kernels, double, order 2 (one translation unit per type and order: they compile side by side)
+#include "wave3d_tile.cuh"
+
+namespace pgb {
+PGB_INSTANTIATE_3D(double, 1)
+}  // namespace pgb
