@@ -4,7 +4,8 @@
 // together in every launch):
 //   forward sweep   k = 0..n-1: record traces of u_k, step to u_{k+1}; every S
 //                   steps save the step inputs (u_{k-1}, u_k, PML state) as a
-//                   checkpoint            (TemporalModeling.forward_model,
+//                   checkpoint (the last segment may write its dWaveOp_k at once
+//                   instead)              (TemporalModeling.forward_model,
 //                   pysit/modeling/temporal_modeling.py:115-161, without the
 //                   per-step dWaveOp list of :146-148)
 //   residual        r = dobs - dsim and ||r||^2 in FP64
@@ -347,6 +348,14 @@ struct PlanT final : public pysit_plan {
         size_t gpad, partial, rnorm, err, tasks, shsteps;
     } off{};
     size_t field_bytes = 0;      // one field for G shots
+    // Checkpointed gradients.  A launch that fills the GPU runs the last segment of the forward sweep
+    // in recompute mode, straight into the replay buffer (one segment less to recompute).  One that
+    // leaves the GPU idle recomputes a segment beside the adjoint steps of the segment after it, on
+    // a second stream and into a second replay buffer.  (1D and small 3D launches do both; small 2D
+    // launches keep a recompute step for every step.)
+    bool overlap = false, keep_last = false;
+    cudaStream_t aux = nullptr;  // the recompute steps' stream when they overlap
+    cudaEvent_t ev_fork = nullptr, ev_ready[2] = {nullptr, nullptr}, ev_free[2] = {nullptr, nullptr};
     int ckpt_fields = 0;         // fields per checkpoint
     bool model_set = false;
     // ---- graphs ----------------------------------------------------------------
@@ -374,6 +383,9 @@ struct PlanT final : public pysit_plan {
         for (auto& kv : graphs)
             if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
         if (cap) cudaStreamDestroy(cap);
+        if (aux) cudaStreamDestroy(aux);
+        for (auto e : {ev_fork, ev_ready[0], ev_ready[1], ev_free[0], ev_free[1]})
+            if (e) cudaEventDestroy(e);
     }
 
     template <typename U>
@@ -443,6 +455,10 @@ struct PlanT final : public pysit_plan {
         nslots = store_all ? (nsteps + p_img - 1) / p_img : S;
         ckpt_fields = dim == 1 ? 3 : dim == 2 ? 4 : 6;
         choose_tiling();
+        const bool fills = dim == 2 ? strip2d == 4 : dim == 3 && planes3d == 4;
+        const bool ckpt = !store_all && !fwd_only;
+        overlap = ckpt && !fills && nseg > 1;
+        keep_last = ckpt && (fills || dim != 2);
         // acquisition
         int rc = build_injection(d.src_tap_ptr, d.src_tap_cell, d.src_tap_point, d.src_tap_w, nsrc,
                                  src_inj, "source");
@@ -821,8 +837,8 @@ struct PlanT final : public pysit_plan {
         }
         off.ic = take(adj_bytes);
         off.m1 = take(fwd_only ? 0 : one);
-        off.replay = take(fwd_only ? 0 : field_bytes * (size_t)nslots);
-        off.ckpt = take(fwd_only || store_all ? 0 : field_bytes * (size_t)ckpt_fields * nseg);
+        off.replay = take(fwd_only ? 0 : field_bytes * (size_t)nslots * (overlap ? 2 : 1));
+        off.ckpt = take(fwd_only || store_all ? 0 : field_bytes * (size_t)ckpt_fields * (nseg - (keep_last ? 1 : 0)));
         off.traces = take((size_t)G * nsteps * nrec * sizeof(T));
         off.srcamp = take((size_t)nshots * nsteps * nsrc * sizeof(T));
         auto take_inj = [&](std::vector<CSRBox>& v, size_t& box, size_t& rpb, size_t& row, size_t& pt,
@@ -915,6 +931,11 @@ struct PlanT final : public pysit_plan {
         if ((rc = upload(off.shsteps, shot_steps, s))) return rc;
         PGB_CHECK_CUDA(cudaStreamSynchronize(s));
         if (!cap) PGB_CHECK_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
+        if (overlap) {
+            if (!aux) PGB_CHECK_CUDA(cudaStreamCreateWithFlags(&aux, cudaStreamNonBlocking));
+            for (auto e : {&ev_fork, &ev_ready[0], &ev_ready[1], &ev_free[0], &ev_free[1]})
+                if (!*e) PGB_CHECK_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+        }
         if (dim == 3) switch (R) {
             case 1: wave3d_tile_prepare<T, 1>(); break;
             case 2: wave3d_tile_prepare<T, 2>(); break;
@@ -1106,6 +1127,8 @@ struct PlanT final : public pysit_plan {
     }
 
     T* replay_slot(long long i) const { return fld(off.replay) + (size_t)i * fstride * G; }
+    // step k of segment seg in its replay buffer
+    T* replay_seg(int seg, int k) const { return replay_slot((overlap ? (seg & 1) * (long long)S : 0) + k - (long long)seg * S); }
 
     T* ckpt_slot(int seg, int f) const {
         return reinterpret_cast<T*>(ws + off.ckpt + ((size_t)seg * ckpt_fields + f) * field_bytes);
@@ -1118,13 +1141,14 @@ struct PlanT final : public pysit_plan {
         State st = make_state(off.U, off.PX, off.PY, off.PZ, off.PS);
         WaveParams<T> p = base_params(g0, gn);
         T* tr = at<T>(off.traces);
-        const bool keep = checkpoints && store_all;
+        const int last0 = (nseg - 1) * S;  // first step of the last segment
         for (int k = 0; k < nsteps; ++k) {
-            if (keep) {
+            const bool tail = checkpoints && keep_last && k >= last0;
+            if (checkpoints && (store_all || tail)) {
                 bind_state(p, st);
                 set_inject(p, true, g0, k, nullptr);
                 set_recording(p, g0, gn, tr + (long long)k * nrec);
-                p.dw_out = (k % p_img == 0) ? replay_slot(k / p_img) : nullptr;
+                p.dw_out = k % p_img != 0 ? nullptr : tail ? replay_seg(nseg - 1, k) : replay_slot(k / p_img);
                 p.nan_check = 1;
                 launch(p, kRecomp, s);
                 advance(st);
@@ -1163,34 +1187,46 @@ struct PlanT final : public pysit_plan {
             }
             return;
         }
+        cudaStream_t rs = overlap ? aux : s;  // the recompute steps' stream
+        if (overlap) {
+            cudaEventRecord(ev_fork, s);
+            cudaStreamWaitEvent(rs, ev_fork, 0);
+        }
         for (int seg = nseg - 1; seg >= 0; --seg) {
-            const int k0 = seg * S, k1 = std::min(k0 + S, nsteps) - 1;
-            // restore the forward state at k0 into buffer set 0
-            State fw = make_state(off.U, off.PX, off.PY, off.PZ, off.PS);
-            {
+            const int k0 = seg * S, k1 = std::min(k0 + S, nsteps) - 1, b = seg & 1;
+            if (!(keep_last && seg == nseg - 1)) {
+                // the segment's replay buffer is free once the adjoint has read segment seg + 2
+                if (overlap && seg + 2 <= nseg - 1) cudaStreamWaitEvent(rs, ev_free[b], 0);
+                // restore the forward state at k0 into buffer set 0
+                State fw = make_state(off.U, off.PX, off.PY, off.PZ, off.PS);
                 T* dst[6]; T* src[6];
                 ckpt_ptrs(fw, dst);
                 for (int f = 0; f < ckpt_fields; ++f) src[f] = ckpt_slot(seg, f);
-                copy_fields(dst, src, s);
-            }
-            WaveParams<T> p = base_params(g0, gn);
-            for (int k = k0; k <= k1; ++k) {
-                bind_state(p, fw);
-                set_inject(p, true, g0, k, nullptr);
-                p.dw_out = (k % period == 0) ? fld(off.replay) + (size_t)(k - k0) * fstride * G : nullptr;
-                launch(p, kRecomp, s);
-                advance(fw);
+                copy_fields(dst, src, rs);
+                WaveParams<T> p = base_params(g0, gn);
+                for (int k = k0; k <= k1; ++k) {
+                    bind_state(p, fw);
+                    set_inject(p, true, g0, k, nullptr);
+                    p.dw_out = (k % period == 0) ? replay_seg(seg, k) : nullptr;
+                    launch(p, kRecomp, rs);
+                    advance(fw);
+                }
+                if (overlap) {
+                    cudaEventRecord(ev_ready[b], rs);
+                    cudaStreamWaitEvent(s, ev_ready[b], 0);
+                }
             }
             WaveParams<T> q = base_params(g0, gn);
             for (int k = k1; k >= k0; --k) {
                 bind_state(q, adj);
                 set_inject(q, false, g0, k, resid);
                 q.image = (k % period == 0);
-                q.dw_in = fld(off.replay) + (size_t)(k - k0) * fstride * G;
+                q.dw_in = replay_seg(seg, k);
                 q.ic = fld(off.ic);
                 launch(q, kAdj, s);
                 advance(adj);
             }
+            if (overlap) cudaEventRecord(ev_free[b], s);
         }
     }
 
@@ -1210,8 +1246,10 @@ struct PlanT final : public pysit_plan {
         const int nb = (int)std::min<long long>(rows, 152LL * 16);
         for (int k = 0; k < nsteps; ++k) {
             // kept schedule: dWaveOp0 of every step stays for the migration (imaging every step)
-            T* dw = checkpoints && store_all ? replay_slot(k) : replay_slot(0);
-            if (checkpoints && !store_all && k % S == 0) {
+            // (checkpointed: that of the last segment stays, where keep_last)
+            const bool tail = checkpoints && keep_last && k >= (nseg - 1) * S;
+            T* dw = checkpoints && store_all ? replay_slot(k) : tail ? replay_seg(nseg - 1, k) : replay_slot(0);
+            if (checkpoints && !store_all && !tail && k % S == 0) {
                 T* src[6]; T* dst[6];
                 ckpt_ptrs(u0, src);
                 for (int f = 0; f < ckpt_fields; ++f) dst[f] = ckpt_slot(k / S, f);
