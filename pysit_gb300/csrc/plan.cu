@@ -323,6 +323,7 @@ struct PlanT final : public pysit_plan {
     int ntask3d[2] = {0, 0};
     int planes3d = 4;            // 3D: x-planes per thread and round
     int strip2d = 4;             // 2D: x-rows per thread of a tile
+    int threads2d = kT2;         // 2D: threads of a block
     std::vector<Tile2d> tiles2d;      // 2D: the device's form of tasks2d
     int inj_cap[2] = {0, 0};     // 2D, 3D: injection cells of a tile at most (source, receivers)
     double shell_frac[4] = {0.0, 0.0, 0.0, 0.0};  // descriptor's shell shares (read back by tuning(); unused)
@@ -484,6 +485,7 @@ struct PlanT final : public pysit_plan {
             bz = kT2;
             tx = tile_req ? tile_req : 32;
             strip2d = choose_strip2d();
+            threads2d = choose_threads2d();
             build_tasks2d();
             ntz = ntx = 1;
             return;
@@ -515,6 +517,15 @@ struct PlanT final : public pysit_plan {
         const long long threads = (long long)nx * nz * G / (16 / (int)sizeof(T));
         const int full = 4 * 152;  // resident blocks of the GPU
         return threads >= 4LL * kT2 * full ? 4 : threads >= 2LL * kT2 * full / 2 ? 2 : 1;
+    }
+
+    // Threads of a 2D block: fewer where kT2 would leave SMs without two blocks (a small FP64 launch
+    // is bound by the FP64 units of the SMs it runs on).  Measured (us per forward step at 128 / 64 /
+    // 32 threads): 141 x 81 cells FP64 7.1 / 6.6 / 6.0; 1232 x 464 FP32 4.9 / 4.7 / 5.3; 461 x 203 x
+    // 6 shots FP64 75 / 78 / 80
+    int choose_threads2d() const {
+        const long long threads = (long long)nx * nz * G / (16 / (int)sizeof(T)) / strip2d;
+        return threads >= 2LL * 152 * 128 ? kT2 : threads >= 2LL * 152 * 64 ? 64 : 32;
     }
 
     // Tiles covering the padded grid once.  Interior (kind 0): cells at least
@@ -556,7 +567,7 @@ struct PlanT final : public pysit_plan {
         // even x chunks of at most tx rows, whole rounds of the block's strips
         int zw = 0;
         for (auto& z : zs) zw = std::max(zw, z.second - z.first);
-        const int once = wave2d_tile_rows((int)sizeof(T), kind, strip2d, zw);
+        const int once = wave2d_tile_rows((int)sizeof(T), kind, strip2d, threads2d, zw);
         const int rows = std::min(once, tx);
         const int nxc = (xb - xa + rows - 1) / rows;
         const int wx = std::min(rows, ((xb - xa + nxc - 1) / nxc + strip2d - 1) / strip2d * strip2d);
@@ -1025,7 +1036,7 @@ struct PlanT final : public pysit_plan {
         // 64 shots of 1232 x 464 cells (FP32): recompute 175 -> 162, adjoint 248 -> 215 us; two or
         // three shots ahead 162 / 166 and 230 / 257 us
         q.pf_next = p.nshot > 1 && 2 * (size_t)fstride * sizeof(T) * p.nshot > ((size_t)48 << 20);
-        launch_wave2d_tiles<T, RR, MODE>(q, at<Tile2d>(off.tasks), ntask2d[0], ntask2d[1], strip2d,
+        launch_wave2d_tiles<T, RR, MODE>(q, at<Tile2d>(off.tasks), ntask2d[0], ntask2d[1], strip2d, threads2d,
                                          inj_cap[MODE == kAdj], s);
         ++launches;
     }

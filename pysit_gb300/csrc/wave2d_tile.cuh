@@ -277,7 +277,8 @@ __global__ void __launch_bounds__(kT2, (sizeof(T) == 4 ? PGB_T2_MINB : 2))
     int t = (int)blockIdx.x - rec;
     if (t < 0) {  // leading blocks record the traces of u_k, one pass per warp
         const long long n = (long long)gridDim.y * gridDim.z;
-        const long long pass = ((long long)blockIdx.x * n + shot) * (kT2 / 32) + (threadIdx.x >> 5);
+        const long long pass = ((long long)blockIdx.x * n + shot) * (blockDim.x / 32) + (threadIdx.x >> 5);
+        pdl_handover();
         if (MODE != kAdj && pass < record_passes(p)) record_pass(p, pass);
         return;
     }
@@ -287,6 +288,24 @@ __global__ void __launch_bounds__(kT2, (sizeof(T) == 4 ? PGB_T2_MINB : 2))
     const int x0 = t0.x, rows = t0.y, zs = t0.z, ncell = t0.w, nzv = t1.x, inv = t1.y;
     const bool pml = t1.z != 0;
     const int s0 = (threadIdx.x * inv) >> 16, q = threadIdx.x - s0 * nzv, r0 = s0 * RS;
+    // the injection of the tile's cells
+    int4 ib = make_int4(0, 0, 0, 0);
+    T* rhs = reinterpret_cast<T*>(smem_raw);
+    if (MODE != kBorn && p.inj.on) {
+        const int* bx = p.inj.box + shot * 6;
+        const int bx0 = max(__ldg(bx), x0), bx1 = min(__ldg(bx + 1), x0 + rows);
+        const int bz0 = max(__ldg(bx + 4), zs), bz1 = min(__ldg(bx + 5), zs + ncell);
+        if (bx0 < bx1 && bz0 < bz1) {
+            ib = make_int4(bx0, bx1, bz0, bz1);
+            const int w = bz1 - bz0, n = (bx1 - bx0) * w;
+            for (int c = threadIdx.x; c < n; c += blockDim.x) {
+                const int dx = c / w;
+                rhs[c] = inject_rhs(p.inj, bx, shot, bx0 + dx, bz0 + c - dx * w);
+            }
+            __syncthreads();
+        }
+    }
+    pdl_handover();
     // fetch the same tile of the next shot into L2: its block starts about when this one ends
     if (p.pf_next && shot + 1 < p.nshot) {
         const long long org = (long long)(shot + 1) * p.fstride + (long long)(x0 + kHalo) * p.ldz + kOZ + zs;
@@ -304,24 +323,7 @@ __global__ void __launch_bounds__(kT2, (sizeof(T) == 4 ? PGB_T2_MINB : 2))
             if (MODE == kAdj && w == 3) rows_of(p.ic);
         }
     }
-    // the injection of the tile's cells
-    int4 ib = make_int4(0, 0, 0, 0);
-    T* rhs = reinterpret_cast<T*>(smem_raw);
-    if (MODE != kBorn && p.inj.on) {
-        const int* bx = p.inj.box + shot * 6;
-        const int bx0 = max(__ldg(bx), x0), bx1 = min(__ldg(bx + 1), x0 + rows);
-        const int bz0 = max(__ldg(bx + 4), zs), bz1 = min(__ldg(bx + 5), zs + ncell);
-        if (bx0 < bx1 && bz0 < bz1) {
-            ib = make_int4(bx0, bx1, bz0, bz1);
-            const int w = bz1 - bz0, n = (bx1 - bx0) * w;
-            for (int c = threadIdx.x; c < n; c += kT2) {
-                const int dx = c / w;
-                rhs[c] = inject_rhs(p.inj, bx, shot, bx0 + dx, bz0 + c - dx * w);
-            }
-            __syncthreads();
-        }
-    }
-    if (r0 >= rows || s0 >= ((kT2 * inv) >> 16)) return;
+    if (r0 >= rows || s0 >= ((int)(blockDim.x * inv) >> 16)) return;
     using O = PairOps<T>;
     typename O::P chk = O::dup(T(0));  // 0 x every u_{k+1}: a NaN or Inf anywhere leaves a NaN here
     // (the injection is looked at row by row only in tiles that meet the box)
@@ -341,15 +343,15 @@ __global__ void __launch_bounds__(kT2, (sizeof(T) == 4 ? PGB_T2_MINB : 2))
 }  // namespace
 
 template <typename T, int R, int MODE>
-void launch_wave2d_tiles(const WaveParams<T>& p, const Tile2d* tiles, int nint, int nshell, int strip, int inj_cap,
-                         cudaStream_t s) {
+void launch_wave2d_tiles(const WaveParams<T>& p, const Tile2d* tiles, int nint, int nshell, int strip, int threads,
+                         int inj_cap, cudaStream_t s) {
     const int gz = ceil_div(p.nshot, 65535), gy = ceil_div(p.nshot, gz);
     // recorder blocks: one pass per warp, the same number for every shot
     const long long passes = MODE != kAdj && p.rec.traces ? ((long long)p.nshot * p.rec.nrec * p.rec.lanes + 31) / 32 : 0;
-    const int rec = ceil_div(passes, (long long)gy * gz * (kT2 / 32));
+    const int rec = ceil_div(passes, (long long)gy * gz * (threads / 32));
     const dim3 grid(rec + nint + nshell, gy, gz);
     const size_t smem = inj_cap * sizeof(T);
-#define PGB_G(RS) wave2d_tile_kernel<T, R, MODE, RS><<<grid, kT2, smem, s>>>(p, tiles, nint, nshell, rec)
+#define PGB_G(RS) launch_step(wave2d_tile_kernel<T, R, MODE, RS>, grid, dim3(threads), smem, s, p, tiles, nint, nshell, rec)
     switch (strip) {
         case 1: PGB_G(1); break;
         case 2: PGB_G(2); break;
@@ -359,7 +361,7 @@ void launch_wave2d_tiles(const WaveParams<T>& p, const Tile2d* tiles, int nint, 
 }
 
 #define PGB_INST2D(T, R, M) \
-    template void launch_wave2d_tiles<T, R, M>(const WaveParams<T>&, const Tile2d*, int, int, int, int, cudaStream_t);
+    template void launch_wave2d_tiles<T, R, M>(const WaveParams<T>&, const Tile2d*, int, int, int, int, int, cudaStream_t);
 #define PGB_INSTANTIATE_2D(T, R) PGB_INST2D(T, R, kFwd) PGB_INST2D(T, R, kRecomp) PGB_INST2D(T, R, kAdj) PGB_INST2D(T, R, kBorn)
 
 }  // namespace pgb

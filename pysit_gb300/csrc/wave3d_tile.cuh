@@ -777,6 +777,7 @@ __global__ void __launch_bounds__(kT3, (sizeof(T) == 4 ? PGB_T3_MINB : 1))
     if (t < 0) {  // leading blocks record the traces of u_k, one pass per warp
         const long long nb = (long long)gridDim.y * gridDim.z;
         const long long pass = ((long long)blockIdx.x * nb + shot) * (kT3 / 32) + (threadIdx.x >> 5);
+        pdl_handover();
         if (MODE != kAdj && pass < record_passes(p)) record_pass(p, pass);
         return;
     }
@@ -803,6 +804,7 @@ __global__ void __launch_bounds__(kT3, (sizeof(T) == 4 ? PGB_T3_MINB : 1))
             __syncthreads();
         }
     }
+    pdl_handover();
     if (lr >= rpw || j >= y1) return;
     const bool inj_col = ib.meets(j, zl, V);
     const long long sh = (long long)shot * p.fstride;
@@ -882,9 +884,9 @@ void launch_wave3d_tiles(const WaveParams<T>& p, const Tile3d* tiles, int nint, 
     const dim3 grid(rec + nint + nshell, gy, gz);
     const size_t smem = inj_cap * sizeof(T);
     if (planes == 1)
-        wave3d_tile_kernel<T, R, MODE, 1><<<grid, kT3, smem, s>>>(p, tiles, nint, nshell, rec);
+        launch_step(wave3d_tile_kernel<T, R, MODE, 1>, grid, dim3(kT3), smem, s, p, tiles, nint, nshell, rec);
     else
-        wave3d_tile_kernel<T, R, MODE, 4><<<grid, kT3, smem, s>>>(p, tiles, nint, nshell, rec);
+        launch_step(wave3d_tile_kernel<T, R, MODE, 4>, grid, dim3(kT3), smem, s, p, tiles, nint, nshell, rec);
 }
 
 #define PGB_INST3D(T, R, M) \
