@@ -55,6 +55,27 @@ template <> struct PairOps<double> {
         return make_double2(::fma(a.x, b.x, c.x), ::fma(a.y, b.y, c.y));
     }
 };
+// Notices a NaN or Inf among the pairs it is shown: FP32 adds 0 x each (a NaN stays), FP64 looks at
+// the exponents (the FP64 units are what the FP64 kernels wait for)
+template <typename T>
+struct FiniteCheck {
+    using O = PairOps<T>;
+    typename O::P c;
+    unsigned big = 0;
+    __device__ __forceinline__ FiniteCheck() : c(O::dup(T(0))) {}
+    __device__ __forceinline__ void see(typename O::P v) {
+        if constexpr (sizeof(T) == 4) {
+            c = O::fma(v, O::dup(T(0)), c);
+        } else {
+            auto e = [](double a) { return (unsigned)__double2hiint(a) & 0x7fffffffu; };
+            big = max(big, max(e(v.x), e(v.y)));
+        }
+    }
+    __device__ __forceinline__ bool bad() const {
+        if constexpr (sizeof(T) == 4) return !(O::lo(c) + O::hi(c) == T(0));
+        else return big >= 0x7ff00000u;
+    }
+};
 // N pairs of neighbouring cells: a thread's vector along z
 template <typename T, int N>
 struct Pairs {
@@ -74,6 +95,22 @@ __device__ __forceinline__ void ldr(Pairs<float, 2>& r, const float* q) {
 }
 __device__ __forceinline__ void ldr(Pairs<float, 1>& r, const float* q) { r.p[0] = __ldg(reinterpret_cast<const unsigned long long*>(q)); }
 __device__ __forceinline__ void ldr(Pairs<double, 1>& r, const double* q) { r.p[0] = __ldg(reinterpret_cast<const double2*>(q)); }
+__device__ __forceinline__ void ldp(Pairs<double, 2>& r, const double* q) {
+    r.p[0] = reinterpret_cast<const double2*>(q)[0];
+    r.p[1] = reinterpret_cast<const double2*>(q)[1];
+}
+__device__ __forceinline__ void ldr(Pairs<double, 2>& r, const double* q) {
+    r.p[0] = __ldg(reinterpret_cast<const double2*>(q));
+    r.p[1] = __ldg(reinterpret_cast<const double2*>(q) + 1);
+}
+__device__ __forceinline__ void stp(double* q, const Pairs<double, 2>& r) {
+    reinterpret_cast<double2*>(q)[0] = r.p[0];
+    reinterpret_cast<double2*>(q)[1] = r.p[1];
+}
+__device__ __forceinline__ void stp_cs(double* q, const Pairs<double, 2>& r) {
+    __stcs(reinterpret_cast<double2*>(q), r.p[0]);
+    __stcs(reinterpret_cast<double2*>(q) + 1, r.p[1]);
+}
 __device__ __forceinline__ void stp(float* q, const Pairs<float, 2>& r) { *reinterpret_cast<ulonglong2*>(q) = make_ulonglong2(r.p[0], r.p[1]); }
 __device__ __forceinline__ void stp(float* q, const Pairs<float, 1>& r) { *reinterpret_cast<unsigned long long*>(q) = r.p[0]; }
 __device__ __forceinline__ void stp(double* q, const Pairs<double, 1>& r) { *reinterpret_cast<double2*>(q) = r.p[0]; }
@@ -135,12 +172,6 @@ __host__ __device__ constexpr double c1sum(int R, int j) {
     for (int m = j + 1; m <= R; ++m) s += d1w(R, m);
     return s;
 }
-
-template <typename T> __device__ __forceinline__ T rcp_(T x);
-// FP32: the fast reciprocal (within ~1 ulp; the FP32 path's tolerances are 1e-4 / 1e-3);
-// FP64 keeps the exact division of the reference
-template <> __device__ __forceinline__ float rcp_(float x) { return __fdividef(1.0f, x); }
-template <> __device__ __forceinline__ double rcp_(double x) { return 1.0 / x; }
 
 }  // namespace
 }  // namespace pgb

@@ -59,6 +59,12 @@ __device__ __forceinline__ long long ioff(int i, int j, int k, int hx, int hy, i
 }
 
 template <typename T>
+__global__ void one_sigma_kernel(const T* __restrict__ s, int n, int dim, T dt, T dt2, T* __restrict__ out) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        out[i] = one_sigma_fac(dim, dt, dt2, s[i]);
+}
+
+template <typename T>
 __global__ void set_c2_kernel(const double* __restrict__ C, int nx, int ny, int nz, int hx,
                               int hy, int rows_y, int ldz, T* __restrict__ c2) {
     long long n = (long long)nx * ny * nz;
@@ -322,6 +328,7 @@ struct PlanT final : public pysit_plan {
     std::vector<Tile3d> tiles3d; // 3D: the device's form of tasks3d
     int ntask3d[2] = {0, 0};
     int planes3d = 4;            // 3D: x-planes per thread and round
+    int threads3d = kT3;         // 3D: threads of a block
     int strip2d = 4;             // 2D: x-rows per thread of a tile
     int threads2d = kT2;         // 2D: threads of a block
     std::vector<Tile2d> tiles2d;      // 2D: the device's form of tasks2d
@@ -339,7 +346,7 @@ struct PlanT final : public pysit_plan {
     char* ws = nullptr;
     uint64_t ws_need = 0;
     struct Off {
-        size_t c2, sgx, sgy, sgz, mgx, mgy, mgz;
+        size_t c2, sgx, sgy, sgz, mgx, mgy, mgz, fcx, fcy, fcz;
         size_t U[2], PX[2], PY[2], PZ[2], PS[2];   // forward state
         size_t A[2], AX[2], AY[2], AZ[2], AS[2];   // adjoint state
         size_t ic, replay, ckpt, traces, srcamp, m1;
@@ -456,7 +463,7 @@ struct PlanT final : public pysit_plan {
         nslots = store_all ? (nsteps + p_img - 1) / p_img : S;
         ckpt_fields = dim == 1 ? 3 : dim == 2 ? 4 : 6;
         choose_tiling();
-        const bool fills = dim == 2 ? strip2d == 4 : dim == 3 && planes3d == 4;
+        const bool fills = dim == 2 ? (long long)nx * nz * G * (int)sizeof(T) >= 64LL * kT2 * 4 * 152 : dim == 3 && planes3d == 4;
         const bool ckpt = !store_all && !fwd_only;
         overlap = ckpt && !fills && nseg > 1;
         keep_last = ckpt && (fills || dim != 2);
@@ -508,15 +515,16 @@ struct PlanT final : public pysit_plan {
         ntx = (nx + tx - 1) / tx;
     }
 
-    // x-rows per thread of the 2D tiles.  Four rows share the most loads, but make the fewest
-    // threads: a launch too small to give every SM its resident blocks at four rows takes two, and
-    // one below that.  Measured (us per step at 4 / 2 / 1 rows): FP32 1232 x 464 x 64 shots 162 / 209
-    // / 236, x 4 13.0 / 14.0 / 16.0, x 1 (279 blocks at four rows) 5.9 / 5.4 / 5.4; FP64 461 x 203 x 6
-    // (548) 92 / 78 / 80; FP64 141 x 81 x 1 (11) 21 / 12.5 / 7.8
+    // x-rows per thread of the 2D tiles.  More rows share more loads, but make fewer threads: a launch
+    // too small to give every SM its resident blocks at the most rows takes fewer.  FP64 takes two at
+    // most (more rows leave too few blocks to keep the FP64 units busy).  Measured (us per forward step
+    // at 4 / 2 / 1 rows): FP32 1232 x 464 x 64 shots 162 / 209 / 236, x 4 13.0 / 14.0 / 16.0, x 1 (279
+    // blocks at four rows) 5.9 / 5.4 / 5.4; FP64 461 x 203 x 40 shots 361 / 360 / 398, x 6 70 / 61 / 65;
+    // 324 x 224 x 9 46 / 40 / 40; 141 x 81 x 1 (11 blocks) 17 / 9 / 5.5
     int choose_strip2d() const {
         const long long threads = (long long)nx * nz * G / (16 / (int)sizeof(T));
-        const int full = 4 * 152;  // resident blocks of the GPU
-        return threads >= 4LL * kT2 * full ? 4 : threads >= 2LL * kT2 * full / 2 ? 2 : 1;
+        const int full = 4 * 152;  // resident FP32 blocks of the GPU
+        return sizeof(T) == 4 && threads >= 4LL * kT2 * full ? 4 : threads >= 2LL * kT2 * full / 2 ? 2 : 1;
     }
 
     // Threads of a 2D block: fewer where kT2 would leave SMs without two blocks (a small FP64 launch
@@ -567,7 +575,7 @@ struct PlanT final : public pysit_plan {
         // even x chunks of at most tx rows, whole rounds of the block's strips
         int zw = 0;
         for (auto& z : zs) zw = std::max(zw, z.second - z.first);
-        const int once = wave2d_tile_rows((int)sizeof(T), kind, strip2d, threads2d, zw);
+        const int once = wave2d_tile_rows(kind, strip2d, threads2d, zw);
         const int rows = std::min(once, tx);
         const int nxc = (xb - xa + rows - 1) / rows;
         const int wx = std::min(rows, ((xb - xa + nxc - 1) / nxc + strip2d - 1) / strip2d * strip2d);
@@ -604,8 +612,11 @@ struct PlanT final : public pysit_plan {
         tiles2d.clear();
         for (size_t t = 0; t < tasks2d.size(); t += 5) {
             const int rows = tasks2d[t + 1] - tasks2d[t], nc = tasks2d[t + 3] - tasks2d[t + 2], kind = tasks2d[t + 4];
-            const int V = wave2d_cells((int)sizeof(T), kind), nzv = (nc + V - 1) / V;
-            tiles2d.push_back({tasks2d[t], rows, tasks2d[t + 2], nc, nzv, (65536 + nzv - 1) / nzv, kind, 0});
+            const int V = wave2d_cells(kind), nzv = (nc + V - 1) / V;
+            bool xoff = true;  // no sigma along x in the tile's rows
+            for (int x = tasks2d[t]; x < tasks2d[t + 1]; ++x) xoff &= sg[0][x] == 0.0 && mg[0][x] == 0.0;
+            tiles2d.push_back({tasks2d[t], rows, tasks2d[t + 2], nc, nzv, (65536 + nzv - 1) / nzv,
+                               kind && xoff ? 2 : kind, 0});
         }
     }
     void build_tasks2d_() {
@@ -627,16 +638,19 @@ struct PlanT final : public pysit_plan {
 
     // Planes per thread and round, and the default task length, of the 3D tiles: four planes share
     // the most loads, and longer tiles the planes that successive rounds meet in L1, but both make
-    // fewer blocks; a launch keeps about four waves of the GPU's 304 resident blocks.  Measured
+    // fewer blocks; a launch keeps about four waves of the GPU's 608 resident blocks.  Measured
     // (us per forward step, planes x length): 440 x 440 x 340 order 8 FP32 4x32 515 (adjoint 709),
-    // 4x16 520 (691), 4x8 535 (684), 4x64 542 (750), 1x8 616; 121 x 107 x 95 order 4 FP32 x 4 shots 4x4 101, 4x8 103, 4x16 122, 1x4 106;
-    // 53 x 49 x 45 order 4 FP64 x 2 shots 1x1 72, 1x4 91, 4x4 86, 4x16 133
+    // 4x16 520 (691), 4x8 535 (684), 4x64 542 (750), 1x8 616; 121 x 107 x 95 order 4 FP32 x 4 shots 4x4
+    // 101, 4x8 103, 4x16 122, 1x4 106; 53 x 49 x 45 order 4 FP64 x 2 shots 1x1 72, 1x4 91, 4x4 86, 4x16
+    // 133 (all with 256-thread blocks; with 128 / 64 threads 520 -> 492 / 500, 91 -> 79 / 80 and, at one
+    // plane in FP64, 62 -> 50 / 49)
     void choose_tile3d() {
-        const long long blocks = (long long)nx * ny * nz * G / (kT3 * (16 / (int)sizeof(T)));  // of one plane each
+        const long long blocks = (long long)nx * ny * nz * G / (256 * (16 / (int)sizeof(T)));  // 256 threads, one plane
         planes3d = blocks >= 4 * 304 ? 4 : 1;
         tx = 1;
         if (planes3d > 1)
             for (tx = 4; tx < 16 && blocks / (2 * tx) >= 4 * 304; tx *= 2) {}
+        threads3d = planes3d > 1 ? kT3 : 64;
         if (tile_req) tx = tile_req;
     }
 
@@ -657,7 +671,7 @@ struct PlanT final : public pysit_plan {
         for (int x = xa; x < xb; x += wx)
             for (auto& z : zs) {
                 const int nzv = (z.second - z.first + V - 1) / V;
-                for (int y = ya, rows = wave3d_task_rows((int)sizeof(T), z.second - z.first); y < yb; y += rows) {
+                for (int y = ya, rows = wave3d_task_rows((int)sizeof(T), threads3d, z.second - z.first); y < yb; y += rows) {
                     int t[6] = {x, std::min(xb, x + wx), y, std::min(yb, y + rows), z.first, z.second};
                     tasks3d.insert(tasks3d.end(), t, t + 6);
                     tiles3d.push_back({t[0], t[1], t[2], t[3], t[4], t[5], kind, (65536 + nzv - 1) / nzv});
@@ -833,6 +847,7 @@ struct PlanT final : public pysit_plan {
         off.c2 = take(one);
         off.sgx = take(nx * sizeof(T)); off.sgy = take(ny * sizeof(T)); off.sgz = take(nz * sizeof(T));
         off.mgx = take(nx * sizeof(T)); off.mgy = take(ny * sizeof(T)); off.mgz = take(nz * sizeof(T));
+        off.fcx = take(nx * sizeof(T)); off.fcy = take(ny * sizeof(T)); off.fcz = take(nz * sizeof(T));
         // a forward-only plan aliases the adjoint state onto the forward one and keeps
         // no imaging, replay or checkpoint storage
         const size_t adj_bytes = fwd_only ? 0 : field_bytes;
@@ -942,6 +957,12 @@ struct PlanT final : public pysit_plan {
         if ((rc = upload(off.shsteps, shot_steps, s))) return rc;
         PGB_CHECK_CUDA(cudaStreamSynchronize(s));
         if (!cap) PGB_CHECK_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
+        auto one_sigma = [&](size_t sigma, size_t out, int n) {
+            one_sigma_kernel<T><<<grid_for(n, 256), 256, 0, s>>>(at<T>(sigma), n, dim, T(dt), T(dt * dt), at<T>(out));
+        };
+        one_sigma(off.sgx, off.fcx, nx);
+        one_sigma(off.sgy, off.fcy, ny);
+        one_sigma(off.sgz, off.fcz, nz);
         if (overlap) {
             if (!aux) PGB_CHECK_CUDA(cudaStreamCreateWithFlags(&aux, cudaStreamNonBlocking));
             for (auto e : {&ev_fork, &ev_ready[0], &ev_ready[1], &ev_free[0], &ev_free[1]})
@@ -990,6 +1011,7 @@ struct PlanT final : public pysit_plan {
         p.hx = hx; p.hy = hy; p.tx = tx; p.ty = 1; p.ntz = ntz; p.nty = 1; p.ntx = ntx; p.nshot = gn;
         p.c2 = at<T>(off.c2);
         p.sgx = at<T>(off.sgx); p.sgy = at<T>(off.sgy); p.sgz = at<T>(off.sgz);
+        p.fcx = at<T>(off.fcx); p.fcy = at<T>(off.fcy); p.fcz = at<T>(off.fcz);
         p.mgx = at<T>(off.mgx); p.mgy = at<T>(off.mgy); p.mgz = at<T>(off.mgz);
         p.pxl = pl[0]; p.pxr = pr[0]; p.pyl = pl[1]; p.pyr = pr[1]; p.pzl = pl[2]; p.pzr = pr[2];
         p.dt = T(dt); p.dt2 = T(dt * dt); p.idt2 = T(1.0 / (dt * dt)); p.i2dt = T(1.0 / (2.0 * dt));
@@ -1050,7 +1072,7 @@ struct PlanT final : public pysit_plan {
         WaveParams<T> q = p;
         const bool scatter = MODE == kAdj && q.inj.on && inj_cap[1] > 4 * kT3;
         if (scatter) q.inj.on = 0;
-        launch_wave3d_tiles<T, RR, MODE>(q, at<Tile3d>(off.tasks), ntask3d[0], ntask3d[1], planes3d,
+        launch_wave3d_tiles<T, RR, MODE>(q, at<Tile3d>(off.tasks), ntask3d[0], ntask3d[1], planes3d, threads3d,
                                          scatter ? 0 : inj_cap[MODE == kAdj], s);
         ++launches;
         if (scatter) {

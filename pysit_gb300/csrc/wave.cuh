@@ -127,6 +127,7 @@ struct WaveParams {
     // PML (kernel convention) and mesh sigma maps, full length per axis
     const T *sgx, *sgy, *sgz;
     const T *mgx, *mgy, *mgz;
+    const T *fcx, *fcy, *fcz;  // 2 dt^2 / (2 + dt s) of each axis' step sigmas alone (one_sigma_fac)
     int pxl, pxr, pyl, pyr, pzl, pzr;  // padding widths holding PML state
     // scalars
     T dt, dt2, idt2, i2dt, idx, idx2, idy, idy2, idz, idz2;
@@ -146,6 +147,17 @@ struct WaveParams {
     int psi_c2;              // 3D: 1 = C^2 multiplies sigma_x sigma_y sigma_z psi (the reference), 0 = not
     int nan_check;           // kRecomp: flag non-finite u_{k+1} as kFwd does (a forward sweep that keeps dWaveOp)
 };
+
+template <typename T> __device__ __forceinline__ T rcp_(T x);
+// FP32: the fast reciprocal (within ~1 ulp; the FP32 path's tolerances are 1e-4 / 1e-3);
+// FP64 keeps the exact division of the reference
+template <> __device__ __forceinline__ float rcp_(float x) { return __fdividef(1.0f, x); }
+template <> __device__ __forceinline__ double rcp_(double x) { return 1.0 / x; }
+// 2 dt^2 / (2 + dt s) with the rounding of the 2D (product with the reciprocal) and 3D (quotient) updates
+template <typename T>
+__device__ __forceinline__ T one_sigma_fac(int dim, T dt, T dt2, T s) {
+    return dim == 2 ? (T(2) * dt2) * rcp_(::fma(dt, s, T(2))) : T(2) * dt2 / ::fma(dt, s, T(2));
+}
 
 // ---- helpers shared by the 2D kernels ---------------------------------------
 // Programmatic dependent launch: consecutive step kernels of a stream.  A step kernel waits for the
@@ -259,7 +271,7 @@ __device__ __forceinline__ void record_pass(const WaveParams<T>& p, long long pa
 // tiles first
 struct Tile2d {
     int x0, rows, zs, ncell;    // rows x0 .. x0+rows-1, cells zs .. zs+ncell-1
-    int nzv, inv, kind, pad;    // vectors along z, ceil(2^16 / nzv), 0 interior / 1 PML shell
+    int nzv, inv, kind, pad;    // vectors along z, ceil(2^16 / nzv), 0 interior / 1 PML shell / 2 shell, sigma_x zero
 };
 constexpr int kT2 = 128;  // threads of a block at most
 // `strip`: x-rows per thread (1, 2 or 4); `threads`: of a block (32, 64 or kT2); `inj_cap`: cells of
@@ -267,14 +279,14 @@ constexpr int kT2 = 128;  // threads of a block at most
 template <typename T, int R, int MODE>
 void launch_wave2d_tiles(const WaveParams<T>& p, const Tile2d* tiles, int nint, int nshell, int strip, int threads,
                          int inj_cap, cudaStream_t s);
-// cells of a thread along z: a 16-byte vector; an FP32 shell thread takes two cells (its two
-// column and two window sets of registers are twice the interior's)
-constexpr int wave2d_cells(int dtype_bytes, int pml) { return dtype_bytes == 4 && !pml ? 4 : 2; }
-// widest z-range of a tile of each kind: 32 threads
-constexpr int wave2d_seg(int dtype_bytes, int pml) { return 32 * wave2d_cells(dtype_bytes, pml); }
+// cells of a thread along z: four (FP32 a 16-byte vector; FP64 two, whose window of first differences
+// serves all four), two in the shell (two sets of columns and windows to hold)
+constexpr int wave2d_cells(int pml) { return pml ? 2 : 4; }
+// widest z-range of a tile of each kind: 32 16-byte vectors (FP32 shell: 8-byte ones)
+constexpr int wave2d_seg(int dtype_bytes, int pml) { return dtype_bytes == 4 && !pml ? 128 : 64; }
 // x-rows a block's threads take side by side, `strip` rows each
-constexpr int wave2d_tile_rows(int dtype_bytes, int pml, int strip, int threads, int zcells) {
-    const int V = wave2d_cells(dtype_bytes, pml);
+constexpr int wave2d_tile_rows(int pml, int strip, int threads, int zcells) {
+    const int V = wave2d_cells(pml);
     return threads / ((zcells + V - 1) / V) * strip;
 }
 // 3D tiles of one shot, shared by all shots: the device's form of the task table, interior
@@ -283,21 +295,21 @@ struct Tile3d {
     int x0, x1, y0, y1;     // planes and rows
     int zs, ze, kind, inv;  // cells along z; 0 interior, 1 general shell, 2-4 faces; ceil(2^16 / vectors along z)
 };
-constexpr int kT3 = 256;                 // threads of a block
+constexpr int kT3 = 128;                 // threads of a block at most
 constexpr int kMaxInj3d = 160 * 1024;    // bytes of injection cells of a tile at most
-// `planes`: x-planes per thread and round (1 or 4); `inj_cap`: cells of the largest tile's part of
+// `planes`: x-planes per thread and round (1 or 4); `threads`: of a block (64 or kT3); `inj_cap`: cells of the largest tile's part of
 // any shot's injection box
 template <typename T, int R, int MODE>
-void launch_wave3d_tiles(const WaveParams<T>& p, const Tile3d* tiles, int nint, int nshell, int planes, int inj_cap,
-                         cudaStream_t s);
+void launch_wave3d_tiles(const WaveParams<T>& p, const Tile3d* tiles, int nint, int nshell, int planes, int threads,
+                         int inj_cap, cudaStream_t s);
 template <typename T, int R>
 void wave3d_tile_prepare();
 // widest z-range of a tile: 32 vectors
 constexpr int wave3d_seg(int dtype_bytes) { return 32 * (16 / dtype_bytes); }
 // y-rows of a tile of zcells z-cells: a warp takes 32 / vectors rows
-constexpr int wave3d_task_rows(int dtype_bytes, int zcells) {
+constexpr int wave3d_task_rows(int dtype_bytes, int threads, int zcells) {
     const int V = 16 / dtype_bytes;
-    return kT3 / 32 * (32 / ((zcells + V - 1) / V));
+    return threads / 32 * (32 / ((zcells + V - 1) / V));
 }
 template <typename T, int R, int MODE>
 void launch_wave1d(const WaveParams<T>& p, int bz, cudaStream_t s);

@@ -29,7 +29,9 @@
 //   kind 0  interior: at least R cells away from the padding and off the outer
 //           (Dirichlet) ring, no PML state, no masks;
 //   kind 1  PML shell: the padding and its R-wide rim, Phi_x / Phi_z carried where both
-//           sigmas vanish as in the reference.
+//           sigmas vanish as in the reference;
+//   kind 2  PML shell tiles without sigma_x (the z-bands): the update's sigma terms are
+//           per-column constants.
 // The arithmetic runs on cell pairs (packed f32x2 instructions in FP32).
 // Measured against the persistent warps with shared-memory row rings this kernel replaces
 // (us per step, before -> now): 1232 x 464 cells, order 8, FP32, 1 shot 33.9 -> 5.4, 16 shots
@@ -47,14 +49,15 @@ namespace {
 
 // One thread's strip of a tile: RS consecutive x-rows of one vector along z, operands read
 // straight from global memory (L1 serves the rows and vectors that neighbouring threads share).
-template <typename T, int R, int MODE, int RS, bool PML, bool INJ>
+template <typename T, int R, int MODE, int RS, int KIND, bool INJ>
 __device__ __forceinline__ void tile_update(const WaveParams<T>& p, const T* rhs, const int shot, const int x0,
                                             const int rows, const int zs, const int r0, const int q, const int4 ib,
-                                            typename PairOps<T>::P& chk) {
+                                            FiniteCheck<T>& chk) {
     using O = PairOps<T>;
     using P = typename O::P;
-    constexpr int V = wave2d_cells((int)sizeof(T), PML);
-    constexpr int AL = V16<T>::N, HZ = (R + AL - 1) / AL * AL, NB = HZ / V;
+    constexpr bool PML = KIND != 0;
+    constexpr int V = wave2d_cells(PML);
+    constexpr int AL = V > V16<T>::N ? V : V16<T>::N, HZ = (R + AL - 1) / AL * AL, NB = HZ / V;
     constexpr int NP = V / 2, C0 = NB * V;
     constexpr bool DIFF = sizeof(T) == 8;  // FP64: derivatives over first differences (fewest FP64 instructions)
     const int zl = zs + q * V;
@@ -80,8 +83,22 @@ __device__ __forceinline__ void tile_update(const WaveParams<T>& p, const T* rhs
     const int ldz = p.ldz;
     const long long o0 = (long long)(x0 + r0 + kHalo) * ldz + kOZ + zl;  // the strip's first cell in a field
     const T* u = p.u_cur + sh + o0;
+    // what the update of a column needs of sigma_z where sigma_x is zero
+    P zdt[NP], zkx[NP], zkz[NP], zfac[NP], zsi[NP], zds[NP];
+    if (KIND == 2) {
+#pragma unroll
+        for (int k = 0; k < NP; ++k) {
+            const P S = O::mk(sgz[2 * k], sgz[2 * k + 1]);
+            zdt[k] = O::mul(O::dup(p.dt), S);
+            zkx[k] = O::mul(zdt[k], O::dup(p.idx));
+            zkz[k] = O::mul(O::sub(O::dup(T(0)), zdt[k]), O::dup(p.idz));
+            zfac[k] = O::mk(__ldg(p.fcz + min(zl + 2 * k, p.nz - 1)), __ldg(p.fcz + min(zl + 2 * k + 1, p.nz - 1)));
+            zsi[k] = O::mul(S, O::dup(p.i2dt));
+            zds[k] = O::mul(O::sub(O::mk(mgz[2 * k], mgz[2 * k + 1]), S), O::dup(p.i2dt));
+        }
+    }
     T sxr[RS], mxr[RS];
-    if (PML) {
+    if (KIND == 1) {
 #pragma unroll
         for (int r = 0; r < RS; ++r) {
             const int x = min(x0 + r0 + r, p.nx - 1);
@@ -122,8 +139,10 @@ __device__ __forceinline__ void tile_update(const WaveParams<T>& p, const T* rhs
             T sx = T(0), mgx = T(0);
             if (PML) {
                 wp.load(p.phz_in + sh + o - HZ, nullptr);
-                sx = sxr[r];
-                mgx = mxr[r];
+                if (KIND == 1) {
+                    sx = sxr[r];
+                    mgx = mxr[r];
+                }
             }
             T rh[V];
             const bool inj_row = injz && xr >= ib.x && xr < ib.y;
@@ -149,17 +168,19 @@ __device__ __forceinline__ void tile_update(const WaveParams<T>& p, const T* rhs
                 // of the large cancellation of w_0 u_0 (the FP32 path depends on this)
                 // (x and z accumulate separately: two short dependency chains)
                 P Fx = O::dup(T(0)), Fz = Fx;
+                if (DIFF) {  // one chain: an FP64 addition less
 #pragma unroll
-                for (int d = 1; d <= R; ++d) {
-                    if (DIFF) {
-                        Fx = O::fma(wx[d], O::sub(ex(d - 1), ex(-d)), Fx);
-                        Fz = O::fma(wz[d], O::sub(ez(d - 1), ez(-d)), Fz);
-                    } else {
+                    for (int d = R; d >= 1; --d) Fz = O::fma(wx[d], O::sub(ex(d - 1), ex(-d)), Fz);
+#pragma unroll
+                    for (int d = R; d >= 1; --d) Fz = O::fma(wz[d], O::sub(ez(d - 1), ez(-d)), Fz);
+                } else {
+#pragma unroll
+                    for (int d = 1; d <= R; ++d) {
                         Fx = O::fma(wx[d], O::add(O::sub(cv[R + r + d].p[k], uc), O::sub(cv[R + r - d].p[k], uc)), Fx);
                         Fz = w.d2(Fz, wz[d], c, d);
                     }
                 }
-                P F = O::add(Fx, Fz);
+                P F = DIFF ? Fz : O::add(Fx, Fz);
                 if (MODE != kAdj && inj_row) F = O::add(F, O::mk(rh[2 * k], rh[2 * k + 1]));
                 if (MODE == kBorn) F = O::sub(F, O::mul(ici.p[k], dwi.p[k]));  // rhs = -m1 dWaveOp0
                 const P uo = um[r].p[k], c2 = cc[r].p[k];
@@ -177,17 +198,24 @@ __device__ __forceinline__ void tile_update(const WaveParams<T>& p, const T* rhs
                     F = O::add(F, O::fma(dpx, O::dup(p.idx), O::mul(dpz, O::dup(p.idz))));
                     // split-field PML update (_2D.h:157-170), branch-free: with both sigmas
                     // zero it reduces to the plain leapfrog update and carries Phi unchanged
+                    const P phx = px[R + r].p[k], phz = wp.at(c), c2F = O::mul(c2, F);
+                    if (KIND == 2) {  // the same with sigma_x zero, its terms left out
+                        pxo.p[k] = O::fma(zkx[k], dx1, phx);
+                        pzo.p[k] = O::fma(zkz[k], dz1, O::fma(zdt[k], O::mul(phz, O::dup(T(-1))), phz));
+                        P fac2 = O::fma(O::fma(O::dup(T(-2)), uc, uo), O::dup(-p.idt2), c2F);
+                        fac2 = O::fma(zsi[k], uo, fac2);
+                        unew = O::mul(zfac[k], fac2);
+                        if (MODE == kRecomp) d = O::fma(zds[k], O::sub(unew, uo), c2F);
+                    } else {
                     const P szp = O::mk(sgz[2 * k], sgz[2 * k + 1]);
                     const P dsx = O::dup(p.dt * sx), dsz = O::mul(O::dup(p.dt), szp);
                     const P S = O::add(O::dup(sx), szp);  // sx + sz
-                    const P phx = px[R + r].p[k], phz = wp.at(c);
                     // Phi' = Phi - dt s Phi + dt (s_other - s) du/dn
                     pxo.p[k] = O::fma(O::mul(O::sub(dsz, dsx), O::dup(p.idx)), dx1, O::fma(dsx, O::mul(phx, O::dup(T(-1))), phx));
                     pzo.p[k] = O::fma(O::mul(O::sub(dsx, dsz), O::dup(p.idz)), dz1, O::fma(dsz, O::mul(phz, O::dup(T(-1))), phz));
                     // u' = 2 dt^2 / (2 + dt S) * (C^2 F - (u_{k-1} - 2u)/dt^2 + S u_{k-1}/(2dt) - sx sz u)
                     const P den = O::fma(O::dup(p.dt), S, O::dup(T(2)));
                     const P fac1 = O::mul(O::dup(T(2) * p.dt2), O::mk(rcp_(O::lo(den)), rcp_(O::hi(den))));
-                    const P c2F = O::mul(c2, F);
                     P fac2 = O::fma(O::fma(O::dup(T(-2)), uc, uo), O::dup(-p.idt2), c2F);
                     fac2 = O::fma(O::mul(S, O::dup(p.i2dt)), uo, fac2);
                     fac2 = O::fma(O::mul(O::dup(-sx), szp), uc, fac2);
@@ -199,6 +227,7 @@ __device__ __forceinline__ void tile_update(const WaveParams<T>& p, const T* rhs
                         const P dP = O::sub(O::mul(O::dup(mgx), mzp), O::mul(O::dup(sx), szp));
                         d = O::fma(O::mul(dS, O::dup(p.i2dt)), O::sub(unew, uo), c2F);
                         d = O::fma(dP, uc, d);
+                    }
                     }
                 } else {
                     // u_{k+1} = dt^2 C^2 F - (u_{k-1} - 2 u_k)
@@ -237,7 +266,7 @@ __device__ __forceinline__ void tile_update(const WaveParams<T>& p, const T* rhs
             }
             if (MODE == kFwd || MODE == kBorn || (MODE == kRecomp && p.nan_check)) {
 #pragma unroll
-                for (int k = 0; k < NP; ++k) chk = O::fma(un.p[k], O::dup(T(0)), chk);
+                for (int k = 0; k < NP; ++k) chk.see(un.p[k]);
             }
             stp(p.u_prev + sh + o, un);
             if (PML) {
@@ -286,7 +315,8 @@ __global__ void __launch_bounds__(kT2, (sizeof(T) == 4 ? PGB_T2_MINB : 2))
     t = t < nshell ? nint + t : t - nshell;  // the table holds the interior tiles first
     const int4 t0 = __ldg(reinterpret_cast<const int4*>(tiles + t)), t1 = __ldg(reinterpret_cast<const int4*>(tiles + t) + 1);
     const int x0 = t0.x, rows = t0.y, zs = t0.z, ncell = t0.w, nzv = t1.x, inv = t1.y;
-    const bool pml = t1.z != 0;
+    const int kind = t1.z;
+    const bool pml = kind != 0;
     const int s0 = (threadIdx.x * inv) >> 16, q = threadIdx.x - s0 * nzv, r0 = s0 * RS;
     // the injection of the tile's cells
     int4 ib = make_int4(0, 0, 0, 0);
@@ -324,20 +354,19 @@ __global__ void __launch_bounds__(kT2, (sizeof(T) == 4 ? PGB_T2_MINB : 2))
         }
     }
     if (r0 >= rows || s0 >= ((int)(blockDim.x * inv) >> 16)) return;
-    using O = PairOps<T>;
-    typename O::P chk = O::dup(T(0));  // 0 x every u_{k+1}: a NaN or Inf anywhere leaves a NaN here
+    FiniteCheck<T> chk;
     // (the injection is looked at row by row only in tiles that meet the box)
     const bool inj = ib.y > ib.x;
-#define PGB_U(PML, INJ) tile_update<T, R, MODE, RS, PML, INJ>(p, rhs, shot, x0, rows, zs, r0, q, ib, chk)
-    if (pml) {
-        if (MODE != kBorn && inj) PGB_U(true, MODE != kBorn);
-        else PGB_U(true, false);
-    } else {
-        if (MODE != kBorn && inj) PGB_U(false, MODE != kBorn);
-        else PGB_U(false, false);
-    }
+#define PGB_U(KIND)                                                                                     \
+    if (MODE != kBorn && inj)                                                                           \
+        tile_update<T, R, MODE, RS, KIND, MODE != kBorn>(p, rhs, shot, x0, rows, zs, r0, q, ib, chk);   \
+    else                                                                                                \
+        tile_update<T, R, MODE, RS, KIND, false>(p, rhs, shot, x0, rows, zs, r0, q, ib, chk);
+    if (kind == 0) { PGB_U(0) }
+    else if (kind == 2) { PGB_U(2) }
+    else { PGB_U(1) }
 #undef PGB_U
-    if (MODE != kAdj && p.err && !(O::lo(chk) + O::hi(chk) == T(0))) atomicOr(p.err, PGB_ERR_NONFINITE);
+    if (MODE != kAdj && p.err && chk.bad()) atomicOr(p.err, PGB_ERR_NONFINITE);
 }
 
 }  // namespace
@@ -355,7 +384,7 @@ void launch_wave2d_tiles(const WaveParams<T>& p, const Tile2d* tiles, int nint, 
     switch (strip) {
         case 1: PGB_G(1); break;
         case 2: PGB_G(2); break;
-        default: PGB_G(4); break;
+        default: PGB_G(sizeof(T) == 4 ? 4 : 2); break;
     }
 #undef PGB_G
 }

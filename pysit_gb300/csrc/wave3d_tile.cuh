@@ -131,7 +131,7 @@ __device__ __forceinline__ T inject_fac(const WaveParams<T>& p, T sx, T sy, T sz
 template <typename T, int R, int MODE>
 __device__ __forceinline__ void general_update(const WaveParams<T>& p, const T* rhs, const InjBox ib, const int shot,
                                                const int x0, const int x1, const int j, const int zl, const int ze,
-                                               T& chk) {
+                                               FiniteCheck<T>& chk) {
     using VT = typename Vec3<T>::type;
     constexpr int V = Vec3<T>::N;
     constexpr int AL = 16 / (int)sizeof(T);
@@ -311,7 +311,11 @@ __device__ __forceinline__ void general_update(const WaveParams<T>& p, const T* 
                 const T nx_ = phx - p.dt * sx * phx + p.dt * (sy + szv - sx) * dux[v] + p.dt * (sy * szv * psx);
                 const T ny_ = phy - p.dt * sy * phy + p.dt * (szv + sx - sy) * duy[v] + p.dt * (szv * sx * psy);
                 const T nz_ = phz - p.dt * szv * phz + p.dt * (sx + sy - szv) * duz[v] + p.dt * (sx * sy * psz);
-                const T fac1 = T(2) * p.dt2 / (T(2) + p.dt * (sx + sy + szv));
+                // (a division only where two sigmas meet: FP64 takes a dozen instructions for it)
+                T fac1;
+                if (sx == T(0) && sy == T(0)) fac1 = __ldg(p.fcz + min(zl + v, p.nz - 1));
+                else if (szv != T(0) || (sx != T(0) && sy != T(0))) fac1 = T(2) * p.dt2 / (T(2) + p.dt * (sx + sy + szv));
+                else fac1 = sx != T(0) ? __ldg(p.fcx + i) : __ldg(p.fcy + j);
                 // the reference multiplies sigma_x sigma_y sigma_z psi by C^2 (_3D.h:219); the
                 // consistent form (psi_c2 = 0) leaves it out, as the matrix operator does
                 const T src = p.psi_c2 ? c2 * (F[v] - (sx * sy * szv) * ps[v]) : c2 * F[v] - (sx * sy * szv) * ps[v];
@@ -368,7 +372,8 @@ __device__ __forceinline__ void general_update(const WaveParams<T>& p, const T* 
         }
         if (MODE == kFwd || (MODE == kRecomp && p.nan_check)) {
 #pragma unroll
-            for (int v = 0; v < V; ++v) chk = ::fma(v < nv ? un[v] : T(0), T(0), chk);
+            for (int v = 0; v < V; v += 2)
+                chk.see(PairOps<T>::mk(v < nv ? un[v] : T(0), v + 1 < nv ? un[v + 1] : T(0)));
         }
     }
 }
@@ -423,7 +428,7 @@ __device__ __forceinline__ void prefetch_planes(const WaveParams<T>& p, const lo
 template <typename T, int R, int MODE, int RX>
 __device__ __forceinline__ void interior_planes(const WaveParams<T>& p, const T* rhs, const InjBox& ib, const bool inj_col,
                                                 const long long sh, const long long o0, const int x, const int n,
-                                                const int j, const int zl, typename PairOps<T>::P& chk) {
+                                                const int j, const int zl, FiniteCheck<T>& chk) {
     using O = PairOps<T>;
     using P = typename O::P;
     constexpr int V = V16<T>::N, NP = V / 2, HZ = (R + V - 1) / V * V, NB = HZ / V, C0 = NB * V;
@@ -512,7 +517,7 @@ __device__ __forceinline__ void interior_planes(const WaveParams<T>& p, const T*
             if (MODE == kAdj && inj_row)
                 un.p[k] = O::mk(::fma(p.dt2 * O::lo(c2), rh[0], O::lo(un.p[k])), ::fma(p.dt2 * O::hi(c2), rh[1], O::hi(un.p[k])));
             if (MODE == kAdj) ico.p[k] = O::fma(uc, dwi.p[k], ici.p[k]);
-            if (MODE == kFwd || (MODE == kRecomp && p.nan_check)) chk = O::fma(un.p[k], O::dup(T(0)), chk);
+            if (MODE == kFwd || (MODE == kRecomp && p.nan_check)) chk.see(un.p[k]);
         }
         stp(p.u_prev + sh + o, un);
         if (MODE == kRecomp && p.dw_out) stp_cs(p.dw_out + sh + o, dwo);
@@ -539,7 +544,7 @@ template <typename T, int R, int MODE, int RX, int AX>
 __device__ __forceinline__ void face_planes(const WaveParams<T>& p, const T* rhs, const InjBox& ib, const bool inj_col,
                                             const FaceCol<T, V16<T>::N / 2>& col, const long long sh, const long long o0,
                                             const int x, const int n, const int j, const int zl,
-                                            typename PairOps<T>::P& chk) {
+                                            FiniteCheck<T>& chk) {
     using O = PairOps<T>;
     using P = typename O::P;
     constexpr int V = V16<T>::N, NP = V / 2, HZ = (R + V - 1) / V * V, NB = HZ / V, C0 = NB * V;
@@ -682,7 +687,7 @@ __device__ __forceinline__ void face_planes(const WaveParams<T>& p, const T* rhs
             Pairs<T, NP> phx, phy, phz, nx_, ny_, nz_;
             ldr(phx, p.phx_in + sh + o);
             ldr(phy, p.phy_in + sh + o);
-            const T f1 = AX == 2 ? T(0) : T(2) * p.dt2 / (T(2) + p.dt * s1);
+            const T f1 = AX == 0 ? __ldg(p.fcx + i) : AX == 1 ? __ldg(p.fcy + j) : T(0);
 #pragma unroll
             for (int k = 0; k < NP; ++k) {
                 phz.p[k] = wz.at(C0 + 2 * k);
@@ -757,12 +762,12 @@ __device__ __forceinline__ void face_planes(const WaveParams<T>& p, const T* rhs
         }
         if (MODE == kFwd || (MODE == kRecomp && p.nan_check))
 #pragma unroll
-            for (int k = 0; k < NP; ++k) chk = O::fma(un.p[k], O::dup(T(0)), chk);
+            for (int k = 0; k < NP; ++k) chk.see(un.p[k]);
     }
 }
 
 #ifndef PGB_T3_MINB
-#define PGB_T3_MINB 2  // resident 8-warp blocks per SM the FP32 register budget aims at (128 registers)
+#define PGB_T3_MINB 4  // resident 4-warp blocks per SM the FP32 register budget aims at (128 registers)
 #endif
 template <typename T, int R, int MODE, int RX>
 __global__ void __launch_bounds__(kT3, (sizeof(T) == 4 ? PGB_T3_MINB : 1))
@@ -776,7 +781,7 @@ __global__ void __launch_bounds__(kT3, (sizeof(T) == 4 ? PGB_T3_MINB : 1))
     int t = (int)blockIdx.x - rec;
     if (t < 0) {  // leading blocks record the traces of u_k, one pass per warp
         const long long nb = (long long)gridDim.y * gridDim.z;
-        const long long pass = ((long long)blockIdx.x * nb + shot) * (kT3 / 32) + (threadIdx.x >> 5);
+        const long long pass = ((long long)blockIdx.x * nb + shot) * (blockDim.x / 32) + (threadIdx.x >> 5);
         pdl_handover();
         if (MODE != kAdj && pass < record_passes(p)) record_pass(p, pass);
         return;
@@ -797,7 +802,7 @@ __global__ void __launch_bounds__(kT3, (sizeof(T) == 4 ? PGB_T3_MINB : 1))
         if (b.x0 < b.x1 && b.y0 < b.y1 && b.z0 < b.z1) {
             ib = b;
             const int w = b.z1 - b.z0, h = (b.y1 - b.y0) * w, n = (b.x1 - b.x0) * h;
-            for (int c = threadIdx.x; c < n; c += kT3) {
+            for (int c = threadIdx.x; c < n; c += blockDim.x) {
                 const int dx = c / h, e = c - dx * h, dy = e / w;
                 rhs[c] = inject_rhs3(p.inj, bx, shot, b.x0 + dx, b.y0 + dy, b.z0 + e - dy * w);
             }
@@ -810,8 +815,7 @@ __global__ void __launch_bounds__(kT3, (sizeof(T) == 4 ? PGB_T3_MINB : 1))
     const long long sh = (long long)shot * p.fstride;
     const long long xs = (long long)p.rows_y * p.ldz;
     const long long oc = ((long long)(x0 + p.hx) * p.rows_y + (j + p.hy)) * p.ldz + kOZ + zl;
-    P chk = O::dup(T(0));  // 0 x every u_{k+1}: a NaN or Inf anywhere leaves a NaN here
-    T chk1 = T(0);
+    FiniteCheck<T> chk;
     if (kind == 0) {
 #pragma unroll 1
         for (int x = x0; x < x1; x += RX) {
@@ -820,7 +824,7 @@ __global__ void __launch_bounds__(kT3, (sizeof(T) == 4 ? PGB_T3_MINB : 1))
                                             zl, chk);
         }
     } else if (kind == 1) {
-        general_update<T, R, MODE>(p, rhs, ib, shot, x0, x1, j, zl, ze, chk1);
+        general_update<T, R, MODE>(p, rhs, ib, shot, x0, x1, j, zl, ze, chk);
     } else {
         constexpr int RF = RX > 2 ? 2 : RX;
         FaceCol<T, NP> col;
@@ -846,7 +850,7 @@ __global__ void __launch_bounds__(kT3, (sizeof(T) == 4 ? PGB_T3_MINB : 1))
         col.need_z = any_nearz || py;
 #pragma unroll
         for (int k = 0; k < NP; ++k)
-            col.fz[k] = O::mk(T(2) * p.dt2 / (T(2) + p.dt * col.sz[2 * k]), T(2) * p.dt2 / (T(2) + p.dt * col.sz[2 * k + 1]));
+            col.fz[k] = O::mk(__ldg(p.fcz + min(zl + 2 * k, p.nz - 1)), __ldg(p.fcz + min(zl + 2 * k + 1, p.nz - 1)));
 #define PGB_F(AX)                                                                                                       \
     _Pragma("unroll 1") for (int x = x0; x < x1; x += RF) {                                                             \
         prefetch_planes<T, R, MODE, true, RF>(p, sh, oc + (long long)(x + RF - x0) * xs, x1 - x - RF);                  \
@@ -858,7 +862,7 @@ __global__ void __launch_bounds__(kT3, (sizeof(T) == 4 ? PGB_T3_MINB : 1))
         else { PGB_F(2); }
 #undef PGB_F
     }
-    if (MODE != kAdj && p.err && !(O::lo(chk) + O::hi(chk) + chk1 == T(0))) atomicOr(p.err, PGB_ERR_NONFINITE);
+    if (MODE != kAdj && p.err && chk.bad()) atomicOr(p.err, PGB_ERR_NONFINITE);
 }
 
 template <typename T, int R, int MODE, int RX>
@@ -875,22 +879,22 @@ void wave3d_tile_prepare() {
 }
 
 template <typename T, int R, int MODE>
-void launch_wave3d_tiles(const WaveParams<T>& p, const Tile3d* tiles, int nint, int nshell, int planes, int inj_cap,
-                         cudaStream_t s) {
+void launch_wave3d_tiles(const WaveParams<T>& p, const Tile3d* tiles, int nint, int nshell, int planes, int threads,
+                         int inj_cap, cudaStream_t s) {
     const int gz = ceil_div(p.nshot, 65535), gy = ceil_div(p.nshot, gz);
     // recorder blocks: one pass per warp, the same number for every shot
     const long long passes = MODE != kAdj && p.rec.traces ? ((long long)p.nshot * p.rec.nrec * p.rec.lanes + 31) / 32 : 0;
-    const int rec = ceil_div(passes, (long long)gy * gz * (kT3 / 32));
+    const int rec = ceil_div(passes, (long long)gy * gz * (threads / 32));
     const dim3 grid(rec + nint + nshell, gy, gz);
     const size_t smem = inj_cap * sizeof(T);
     if (planes == 1)
-        launch_step(wave3d_tile_kernel<T, R, MODE, 1>, grid, dim3(kT3), smem, s, p, tiles, nint, nshell, rec);
+        launch_step(wave3d_tile_kernel<T, R, MODE, 1>, grid, dim3(threads), smem, s, p, tiles, nint, nshell, rec);
     else
-        launch_step(wave3d_tile_kernel<T, R, MODE, 4>, grid, dim3(kT3), smem, s, p, tiles, nint, nshell, rec);
+        launch_step(wave3d_tile_kernel<T, R, MODE, 4>, grid, dim3(threads), smem, s, p, tiles, nint, nshell, rec);
 }
 
 #define PGB_INST3D(T, R, M) \
-    template void launch_wave3d_tiles<T, R, M>(const WaveParams<T>&, const Tile3d*, int, int, int, int, cudaStream_t);
+    template void launch_wave3d_tiles<T, R, M>(const WaveParams<T>&, const Tile3d*, int, int, int, int, int, cudaStream_t);
 #define PGB_INSTANTIATE_3D(T, R)                                         \
     PGB_INST3D(T, R, kFwd) PGB_INST3D(T, R, kRecomp) PGB_INST3D(T, R, kAdj) \
     template void wave3d_tile_prepare<T, R>();
