@@ -356,6 +356,7 @@ struct PlanT final : public pysit_plan {
         size_t gpad, partial, rnorm, err, tasks, shsteps;
     } off{};
     size_t field_bytes = 0;      // one field for G shots
+    bool sweeps1d = false;       // 1D: runs of steps as one launch
     // Checkpointed gradients.  A launch that fills the GPU runs the last segment of the forward sweep
     // in recompute mode, straight into the replay buffer (one segment less to recompute).  One that
     // leaves the GPU idle recomputes a segment beside the adjoint steps of the segment after it, on
@@ -463,6 +464,7 @@ struct PlanT final : public pysit_plan {
         nslots = store_all ? (nsteps + p_img - 1) / p_img : S;
         ckpt_fields = dim == 1 ? 3 : dim == 2 ? 4 : 6;
         choose_tiling();
+        sweeps1d = dim == 1 && wave1d_sweeps<T>(nz, std::max(nsrc, nrec));
         const bool fills = dim == 2 ? (long long)nx * nz * G * (int)sizeof(T) >= 64LL * kT2 * 4 * 152 : dim == 3 && planes3d == 4;
         const bool ckpt = !store_all && !fwd_only;
         overlap = ckpt && !fills && nseg > 1;
@@ -1167,6 +1169,61 @@ struct PlanT final : public pysit_plan {
         return reinterpret_cast<T*>(ws + off.ckpt + ((size_t)seg * ckpt_fields + f) * field_bytes);
     }
 
+    // steps k0, k0 + dir, ... (n of them) of a 1D grid from state st in one launch; st advances.
+    // in: the state's arrays before the first step where they are not st's own (a checkpoint)
+    void sweep1d(const WaveParams<T>& p, State& st, T* const* in, int mode, int k0, int n, int dir, Sweep1d<T> q,
+                 cudaStream_t s) {
+        if (n <= 0) return;
+        T* own[6];
+        ckpt_ptrs(st, own);
+        if (!in) in = own;
+        q.in_prev = in[0]; q.in_cur = in[1]; q.in_phz = in[2];
+        for (int i = 0; i < n; ++i) advance(st);
+        ckpt_ptrs(st, own);
+        q.out_prev = own[0]; q.out_cur = own[1]; q.out_phz = own[2];
+        q.k0 = k0; q.n = n; q.dir = dir;
+        q.npts_max = std::max(nsrc, nrec);
+        q.field_stride = (long long)fstride * G;
+        q.S = S;
+        ++launches;
+#define PGB_S(RR)                                                             \
+    do {                                                                      \
+        if (mode == kFwd) launch_wave1d_sweep<T, RR, kFwd>(p, q, s);          \
+        else if (mode == kRecomp) launch_wave1d_sweep<T, RR, kRecomp>(p, q, s); \
+        else launch_wave1d_sweep<T, RR, kAdj>(p, q, s);                       \
+    } while (0)
+        switch (R) {
+            case 1: PGB_S(1); break;
+            case 2: PGB_S(2); break;
+            case 3: PGB_S(3); break;
+            default: PGB_S(4); break;
+        }
+#undef PGB_S
+    }
+    // the forward (or recompute) steps [k0, k1): dw as in Sweep1d, `record` their traces
+    void forward1d(int g0, int gn, State& st, T* const* in, int k0, int k1, int mode, T* dw, int period, int dw_k0, int dw_div,
+                   bool record, bool ckpt, cudaStream_t s) {
+        WaveParams<T> p = base_params(g0, gn);
+        set_inject(p, true, g0, 0, nullptr);
+        set_recording(p, g0, gn, at<T>(off.traces));
+        Sweep1d<T> q{};
+        q.npts = nsrc;
+        q.traces = record && nrec > 0 ? at<T>(off.traces) : nullptr;
+        q.dw = dw; q.dw_period = period; q.dw_k0 = dw_k0; q.dw_div = dw_div;
+        q.ckpt = ckpt ? ckpt_slot(0, 0) : nullptr;
+        sweep1d(p, st, in, mode, k0, k1 - k0, 1, q, s);
+    }
+    // the adjoint steps k1 .. k0
+    void adjoint1d(int g0, int gn, State& st, int k0, int k1, const T* dw, int period, int dw_k0, int dw_div, cudaStream_t s) {
+        WaveParams<T> p = base_params(g0, gn);
+        set_inject(p, false, g0, 0, at<T>(off.traces));
+        p.ic = fld(off.ic);
+        Sweep1d<T> q{};
+        q.npts = nrec;
+        q.dw = const_cast<T*>(dw); q.dw_period = period; q.dw_k0 = dw_k0; q.dw_div = dw_div;
+        sweep1d(p, st, nullptr, kAdj, k1, k1 - k0 + 1, -1, q, s);
+    }
+
     // forward sweep of one group; with `checkpoints` (a gradient follows) it saves the
     // checkpoints, or with store_all writes dWaveOp of every imaged step instead
     void forward_sweep(int g0, int gn, bool checkpoints, cudaStream_t s) {
@@ -1175,6 +1232,16 @@ struct PlanT final : public pysit_plan {
         WaveParams<T> p = base_params(g0, gn);
         T* tr = at<T>(off.traces);
         const int last0 = (nseg - 1) * S;  // first step of the last segment
+        if (sweeps1d) {
+            if (checkpoints && store_all) {
+                forward1d(g0, gn, st, nullptr, 0, nsteps, kRecomp, replay_slot(0), p_img, 0, p_img, true, false, s);
+                return;
+            }
+            const int cut = checkpoints && keep_last ? last0 : nsteps;
+            forward1d(g0, gn, st, nullptr, 0, cut, kFwd, nullptr, 1, 0, 1, true, checkpoints, s);
+            forward1d(g0, gn, st, nullptr, cut, nsteps, kRecomp, replay_seg(nseg - 1, last0), p_img, last0, 1, true, false, s);
+            return;
+        }
         for (int k = 0; k < nsteps; ++k) {
             const bool tail = checkpoints && keep_last && k >= last0;
             if (checkpoints && (store_all || tail)) {
@@ -1207,6 +1274,10 @@ struct PlanT final : public pysit_plan {
         cudaMemsetAsync(ws + off.ic, 0, field_bytes, s);
         State adj = make_state(off.A, off.AX, off.AY, off.AZ, off.AS);
         const T* resid = at<T>(off.traces);
+        if (store_all && sweeps1d) {
+            adjoint1d(g0, gn, adj, 0, nsteps - 1, replay_slot(0), period, 0, period, s);
+            return;
+        }
         if (store_all) {  // dWaveOp of every imaged step is in the replay buffer already
             WaveParams<T> q = base_params(g0, gn);
             for (int k = nsteps - 1; k >= 0; --k) {
@@ -1235,9 +1306,12 @@ struct PlanT final : public pysit_plan {
                 T* dst[6]; T* src[6];
                 ckpt_ptrs(fw, dst);
                 for (int f = 0; f < ckpt_fields; ++f) src[f] = ckpt_slot(seg, f);
-                copy_fields(dst, src, rs);
+                if (sweeps1d)
+                    forward1d(g0, gn, fw, src, k0, k1 + 1, kRecomp, replay_seg(seg, k0), period, k0, 1, false, false, rs);
+                else
+                    copy_fields(dst, src, rs);
                 WaveParams<T> p = base_params(g0, gn);
-                for (int k = k0; k <= k1; ++k) {
+                for (int k = k0; k <= k1 && !sweeps1d; ++k) {
                     bind_state(p, fw);
                     set_inject(p, true, g0, k, nullptr);
                     p.dw_out = (k % period == 0) ? replay_seg(seg, k) : nullptr;
@@ -1249,8 +1323,9 @@ struct PlanT final : public pysit_plan {
                     cudaStreamWaitEvent(s, ev_ready[b], 0);
                 }
             }
+            if (sweeps1d) adjoint1d(g0, gn, adj, k0, k1, replay_seg(seg, k0), period, k0, 1, s);
             WaveParams<T> q = base_params(g0, gn);
-            for (int k = k1; k >= k0; --k) {
+            for (int k = k1; k >= k0 && !sweeps1d; --k) {
                 bind_state(q, adj);
                 set_inject(q, false, g0, k, resid);
                 q.image = (k % period == 0);

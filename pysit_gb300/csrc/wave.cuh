@@ -311,6 +311,26 @@ constexpr int wave3d_task_rows(int dtype_bytes, int threads, int zcells) {
     const int V = 16 / dtype_bytes;
     return threads / 32 * (32 / ((zcells + V - 1) / V));
 }
+// A run of 1D steps in one launch (wave1d.cu)
+template <typename T>
+struct Sweep1d {
+    const T *in_prev, *in_cur, *in_phz;  // state before the first step (shot 0)
+    T *out_prev, *out_cur, *out_phz;     // and after the last
+    int k0, n, dir;                      // first step, number of steps, +1 or -1
+    int npts, npts_max;                  // injection points of this run; of any run of the plan
+    T* traces;                           // NULL, or the traces of step 0 of shot 0 (rows of p.rec.nrec)
+    T* dw;                               // NULL, or dWaveOp: step k with k % dw_period == 0 in field (k - dw_k0) / dw_div
+    int dw_period, dw_k0, dw_div;
+    T* ckpt;                             // NULL, or the checkpoints: u_{k-1}, u_k, Phi_z of every S-th step
+    int S;
+    long long field_stride;              // elements between fields of a launch's shots
+    int cells, threads;                  // cells per block and threads that step them (set by the launch)
+};
+// whether a grid of nz cells with at most npts injection points runs as sweeps
+template <typename T>
+bool wave1d_sweeps(int nz, int npts);
+template <typename T, int R, int MODE>
+void launch_wave1d_sweep(const WaveParams<T>& p, Sweep1d<T> q, cudaStream_t s);
 template <typename T, int R, int MODE>
 void launch_wave1d(const WaveParams<T>& p, int bz, cudaStream_t s);
 

@@ -1,6 +1,18 @@
 // Batched 1D leapfrog step (forward, recompute, adjoint modes) on the internal zero-halo layout
 // of wave.cuh, for cda_time_scalar_1D (pysit/solvers/constant_density_acoustic/time/scalar/
-// constant_density_acoustic_time_scalar_1D.h:78-130): one thread per cell.
+// constant_density_acoustic_time_scalar_1D.h:78-130).
+//
+// A whole run of steps is one launch: a cluster of up to sixteen blocks per shot holds the shot's
+// wavefields in shared memory, a block's cells one thread each (or a few), and meets once per step
+// at the cluster barrier after writing the cells its neighbours' stencils reach into their halos.
+// Checkpoints, traces, dWaveOp and the image go to and come from global memory as the steps pass.
+// What bounds a step: in FP64 the few FP64 units of the cluster's SMs, then the barrier.  Measured
+// against one launch per step of one thread per cell (800 steps of 799 cells, order 4, FP64, whole
+// gradient call): 6.4 -> 4.0 ms.  Grids too long for a cluster step as before, one launch each.
+#include <cooperative_groups.h>
+
+#include <algorithm>
+
 #include "wave.cuh"
 
 namespace pgb {
@@ -82,7 +94,213 @@ __global__ void __launch_bounds__(256) wave1d_kernel(const WaveParams<T> p, int 
     if (MODE == kAdj && p.image) p.ic[sh + o] += uc * __ldcs(p.dw_in + sh + o);
 }
 
+// ---- many steps in one launch ---------------------------------------------------------
+namespace cg = cooperative_groups;
+constexpr int kH1 = 4;       // halo cells on either side of a block's cells
+constexpr int kThreads1 = 512;  // threads of a block at most
+constexpr int kAmpSteps = 16;  // steps whose injection amplitudes are staged at once
+
+// shared memory of a block: u x 2, Phi_z x 2 (with halos); C^2, sigmas, factor, image; amplitudes;
+// the injection entries of its cells
+template <typename T>
+size_t sweep1d_smem(int cells, int npts) {
+    return sizeof(T) * (4 * (size_t)(cells + 2 * kH1) + 5 * (size_t)cells + (size_t)kAmpSteps * npts) + 2 * sizeof(int) * (size_t)cells;
+}
+
+template <typename T, int R, int MODE>
+__global__ void __launch_bounds__(kThreads1) wave1d_sweep_kernel(const WaveParams<T> p, const Sweep1d<T> q) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = cl.block_rank(), nc = cl.num_blocks();
+    const int shot = blockIdx.x / nc;
+    const int a = rank * q.cells, n = min(q.cells, p.nz - a);  // the block's cells a .. a+n-1
+    const int w = q.cells + 2 * kH1, tid = threadIdx.x, nt = q.threads;  // nt threads step cells, the warps after them record
+    const int rw = (tid - nt) >> 5, nrw = (blockDim.x - nt) >> 5;
+    T* u[2] = {reinterpret_cast<T*>(smem_raw) + kH1, reinterpret_cast<T*>(smem_raw) + w + kH1};  // u[cur], u[cur ^ 1] = u_{k-1} -> u_{k+1}
+    T* ph[2] = {u[0] + 2 * w, u[0] + 3 * w};
+    T* c2 = u[0] + 4 * w - kH1;
+    T *sg = c2 + q.cells, *mg = sg + q.cells, *fc = mg + q.cells, *ic = fc + q.cells, *amp = ic + q.cells;
+    int* e0 = reinterpret_cast<int*>(amp + kAmpSteps * q.npts);
+    int* e1 = e0 + q.cells;
+    const long long sh = (long long)shot * p.fstride + kOZ;
+    const int* bx = p.inj.box + shot * 6;
+    // the state with its halos (zero beyond the grid: the fields' own zero halos)
+    for (int j = tid - kH1; j < n + kH1; j += blockDim.x) {
+        u[0][j] = q.in_cur[sh + a + j];
+        u[1][j] = j >= 0 && j < n ? q.in_prev[sh + a + j] : T(0);
+        ph[0][j] = q.in_phz[sh + a + j];
+        ph[1][j] = T(0);
+    }
+    for (int j = tid; j < n; j += blockDim.x) {
+        const int k = a + j;
+        c2[j] = p.c2[kOZ + k];
+        sg[j] = p.sgz[k];
+        mg[j] = p.mgz[k];
+        fc[j] = p.fcz[k];
+        ic[j] = MODE == kAdj ? p.ic[sh + k] : T(0);
+        const bool in = p.inj.on && bx[0] <= 0 && bx[1] > 0 && k >= bx[4] && k < bx[5];
+        const int* rp = p.inj.rowptr + (in ? p.inj.rpbase[shot] + k - bx[4] : 0);
+        e0[j] = in ? rp[0] : 0;
+        e1[j] = in ? rp[1] : 0;
+    }
+    // the neighbours' halos: cells j < R go to the left block's right halo, cells j >= n-R to the right's left
+    const int nl = q.cells;  // cells of the left neighbour (only the last block may have fewer)
+    T* left = rank > 0 ? cl.map_shared_rank(u[0], rank - 1) : nullptr;
+    T* right = rank + 1 < nc ? cl.map_shared_rank(u[0], rank + 1) : nullptr;
+    const bool ahead = MODE == kAdj && q.dw && n <= nt && tid < n;
+    T dw_next = ahead && q.k0 % q.dw_period == 0
+                    ? __ldcs(q.dw + (long long)((q.k0 - q.dw_k0) / q.dw_div) * q.field_stride + sh + a + tid) : T(0);
+    cl.sync();
+    int cur = 0;
+    for (int i = 0; i < q.n; ++i) {
+        const int k = q.k0 + q.dir * i;
+        const T *uk = u[cur], *pk = ph[cur];
+        T *un = u[cur ^ 1], *pn = ph[cur ^ 1];
+        if (p.inj.on && i % kAmpSteps == 0) {  // the amplitudes of the next steps
+            const T* src = p.inj.amp + (long long)shot * p.inj.amp_sstride;
+            const int m = min(kAmpSteps, q.n - i) * q.npts;
+            for (int c = tid; c < m; c += blockDim.x) {
+                const int r = c / q.npts;
+                amp[c] = src[(long long)(k + q.dir * r) * q.npts + c - r * q.npts];
+            }
+            __syncthreads();
+        }
+        const T* am = amp + (i % kAmpSteps) * q.npts;
+        if (MODE == kFwd && q.ckpt && k % q.S == 0) {  // the step's inputs: u_{k-1}, u_k, Phi_z
+            T* c = q.ckpt + (long long)(k / q.S) * 3 * q.field_stride + sh + a;
+            for (int j = tid; j < n && rw < 0; j += nt) {
+                c[j] = un[j];
+                c[q.field_stride + j] = uk[j];
+                c[2 * q.field_stride + j] = pk[j];
+            }
+        }
+        if (MODE != kAdj && rw >= 0 && q.traces) {
+            // traces of u_k, a warp per receiver, the blocks in turn: the lanes fetch the taps (from the
+            // block that holds their cell), lane by lane they are summed in order
+            for (int r = rank + nc * rw; r < p.rec.nrec; r += nc * nrw) {
+                const long long id = (long long)shot * p.rec.nrec + r;
+                const int lane = tid & 31, e1r = __ldg(p.rec.rowptr + id + 1);
+                T acc = T(0);
+                for (int e = __ldg(p.rec.rowptr + id); e < e1r; e += 32) {
+                    const int m = min(32, e1r - e);
+                    T wt = T(0), v = T(0);
+                    if (lane < m) {
+                        const int cell = (int)(__ldg(p.rec.off + e + lane) - kOZ), b = cell / q.cells;
+                        wt = __ldg(p.rec.w + e + lane);
+                        v = cl.map_shared_rank(u[0], b)[(uk - u[0]) + cell - b * q.cells];
+                    }
+                    for (int t = 0; t < m; ++t)
+                        acc += __shfl_sync(0xffffffffu, wt, t) * __shfl_sync(0xffffffffu, v, t);
+                }
+                if (lane == 0) q.traces[(long long)shot * p.rec.tr_sstride + (long long)k * p.rec.nrec + r] = acc;
+            }
+        }
+        const bool img = q.dw && k % q.dw_period == 0;
+        const long long slot = img ? (long long)((k - q.dw_k0) / q.dw_div) * q.field_stride + sh + a : 0;
+        // dWaveOp of the next imaged step, on its way while this one computes (one cell per thread)
+        T dw_after = T(0);
+        if (MODE == kAdj && ahead && i + 1 < q.n && (k - 1) % q.dw_period == 0)
+            dw_after = __ldcs(q.dw + (long long)((k - 1 - q.dw_k0) / q.dw_div) * q.field_stride + sh + a + tid);
+        for (int j = tid; j < n && rw < 0; j += nt) {
+            const int c = a + j;
+            const T dw = MODE == kAdj && img ? (ahead ? dw_next : __ldcs(q.dw + slot + j)) : T(0);
+            const bool ok = c > 0 && c < p.nz - 1;
+            const T sz = sg[j], uc = uk[j], uo = un[j], cc = c2[j];
+            // Phi_z is zero outside the padding
+            const bool near = c - R < p.pzl || c + R >= p.nz - p.pzr;
+            T F = dd2<T, R>(uk + j, 1) * p.idz2 + (near ? dd1<T, R>(pk + j, 1) : T(0)) * p.idz;
+            if (e1[j] > e0[j]) {
+                T acc = T(0);
+                for (int e = e0[j]; e < e1[j]; ++e) acc += __ldg(p.inj.w + e) * am[__ldg(p.inj.pt + e)];
+                F += acc;
+            }
+            T unew, pnew = T(0);
+            if (sz != T(0)) {
+                const T dudz = dd1<T, R>(uk + j, 1) * p.idz;
+                const T phz = pk[j];
+                pnew = phz - p.dt * sz * (phz + dudz);
+                const T fac2 = cc * F - (uo - T(2) * uc) * p.idt2 + sz * uo * p.i2dt;
+                unew = fc[j] * fac2;
+                if (!ok) { unew = T(0); pnew = T(0); }
+            } else {
+                unew = p.dt2 * cc * F - (uo - T(2) * uc);
+                if (!ok) unew = T(0);
+            }
+            un[j] = unew;
+            pn[j] = pnew;
+            const int at = (int)(un - u[0]) + j, pt = (int)(pn - u[0]) + j;
+            if (left && j < R) {
+                left[at + nl] = unew;
+                left[pt + nl] = pnew;
+            }
+            if (right && j >= n - R) {
+                right[at - n] = unew;
+                right[pt - n] = pnew;
+            }
+            if (MODE == kRecomp && img) {
+                const T d = cc * F + (mg[j] - sz) * (unew - uo) * p.i2dt;
+                __stcs(q.dw + slot + j, ok ? d : T(0));
+            }
+            if (MODE == kAdj && img) ic[j] += uc * dw;
+        }
+        cl.sync();  // the new fields and halos are complete, the old ones free
+        cur ^= 1;
+        dw_next = dw_after;
+    }
+    for (int j = tid; j < n; j += blockDim.x) {
+        q.out_cur[sh + a + j] = u[cur][j];
+        q.out_prev[sh + a + j] = u[cur ^ 1][j];
+        q.out_phz[sh + a + j] = ph[cur][j];
+        if (MODE == kAdj) p.ic[sh + a + j] = ic[j];
+    }
+}
+
+// blocks per shot and cells per block; 0 blocks: the grid or its point sets are too large for a cluster
+template <typename T>
+int sweep1d_shape(int nz, int npts, int* cells) {
+    // a block's cells: in FP64 as few as give a few warps (the FP64 units bound the step: 2.4 us a step at
+    // 100 cells a block, 3.5 at 250, where a launch per step takes 3.0), with sixteen blocks where eight
+    // would hold more than 128 each; in FP32 a block's threads (1.5 us a step from 150 to 2000 cells)
+    const int want = sizeof(T) == 8 ? 64 : 512, most = sizeof(T) == 8 ? 160 : 2048;
+    const int lim = sizeof(T) == 8 && nz > 8 * 128 ? 16 : 8;
+    int nc = std::min(lim, ceil_div(nz, want));
+    for (;; --nc) {
+        *cells = ceil_div(nz, nc);
+        if (nc == 1 || nz - (nc - 1) * *cells >= kH1) break;  // the last block feeds its neighbour's halo
+    }
+    if (*cells > most || sweep1d_smem<T>(*cells, npts) > 200 * 1024) return 0;
+    return nc;
+}
+
 }  // namespace
+
+template <typename T>
+bool wave1d_sweeps(int nz, int npts) {
+    int cells;
+    return sweep1d_shape<T>(nz, npts, &cells) > 0;
+}
+
+template <typename T, int R, int MODE>
+void launch_wave1d_sweep(const WaveParams<T>& p, Sweep1d<T> q, cudaStream_t s) {
+    const int nc = sweep1d_shape<T>(p.nz, q.npts_max, &q.cells);
+    if (!p.inj.on) q.npts = 0;
+    const size_t smem = sweep1d_smem<T>(q.cells, q.npts);
+    if (smem > 48 * 1024)
+        cudaFuncSetAttribute(wave1d_sweep_kernel<T, R, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (nc > 8) cudaFuncSetAttribute(wave1d_sweep_kernel<T, R, MODE>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(nc * p.nshot);
+    q.threads = std::min(kThreads1 - 128, (q.cells + 31) / 32 * 32);
+    cfg.blockDim = dim3(q.threads + (MODE != kAdj && q.traces ? 32 * std::min(4, ceil_div(p.rec.nrec, nc)) : 0));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim = {(unsigned)nc, 1, 1};
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, wave1d_sweep_kernel<T, R, MODE>, p, q);
+}
 
 template <typename T, int R, int MODE>
 void launch_wave1d(const WaveParams<T>& p, int bz, cudaStream_t s) {
@@ -94,7 +312,12 @@ void launch_wave1d(const WaveParams<T>& p, int bz, cudaStream_t s) {
     wave1d_kernel<T, R, MODE><<<grid, tb, 0, s>>>(p, ntile);
 }
 
+template bool wave1d_sweeps<float>(int, int);
+template bool wave1d_sweeps<double>(int, int);
 #define PGB_INST1(T, R)                                                                  \
+    template void launch_wave1d_sweep<T, R, kFwd>(const WaveParams<T>&, Sweep1d<T>, cudaStream_t);    \
+    template void launch_wave1d_sweep<T, R, kRecomp>(const WaveParams<T>&, Sweep1d<T>, cudaStream_t); \
+    template void launch_wave1d_sweep<T, R, kAdj>(const WaveParams<T>&, Sweep1d<T>, cudaStream_t);    \
     template void launch_wave1d<T, R, kFwd>(const WaveParams<T>&, int, cudaStream_t);    \
     template void launch_wave1d<T, R, kRecomp>(const WaveParams<T>&, int, cudaStream_t); \
     template void launch_wave1d<T, R, kAdj>(const WaveParams<T>&, int, cudaStream_t);
