@@ -314,6 +314,14 @@ class _CDATimeScalarCuda:
             self._sig_dev = (key, sig, maps)
         return self._sig_dev[1], self._sig_dev[2]
 
+    def _field_ptr(self, t, i):
+        """Device pointer of field i of a stacked vector (NULL past its end), without the tensor
+        views that slicing makes: they were most of the host time of a small step."""
+        dof = self.mesh.dof(include_bc=True)
+        if not t.is_contiguous():
+            return t.reshape(-1)[i * dof:(i + 1) * dof].data_ptr()
+        return t.data_ptr() + i * dof * t.element_size() if i * dof < t.numel() else 0
+
     def _field_ptrs(self, vec):
         """(u, aux...) device pointers of a device wavefield vector."""
         d = vec.data
@@ -335,11 +343,9 @@ class _CDATimeScalarCuda:
         if isinstance(rhs_k, np.ndarray):
             rhs = torch.as_tensor(np.ascontiguousarray(rhs_k.reshape(-1)), dtype=tdt, device="cuda")
         else:
-            rhs = rhs_k.reshape(-1).to(dtype=tdt)
+            rhs = rhs_k if rhs_k.dtype == tdt and rhs_k.is_contiguous() else rhs_k.reshape(-1).to(dtype=tdt)
         C = self.device_model().to(tdt) if tdt != torch.float64 else self.device_model()
-        dof = self.mesh.dof(include_bc=True)
-        f = lambda t, i: t.reshape(-1)[i * dof:(i + 1) * dof].data_ptr()  # noqa: E731
-        self._launch_step(f, vkm1, vk, out, C, rhs)
+        self._launch_step(self._field_ptr, vkm1, vk, out, C, rhs)
         if host:
             solver_data.kp1.data[:] = out.reshape(-1, 1).cpu().numpy()
 
@@ -356,19 +362,21 @@ class _CDATimeScalarCuda:
         tdt = torch.float64 if self.dtype == np.double else torch.float32
         dof = self.mesh.dof(include_bc=True)
 
-        def dev(v, i=0):
-            d = v.data
-            if host:
-                return torch.as_tensor(np.ascontiguousarray(d[i * dof:(i + 1) * dof].reshape(-1)), dtype=tdt,
+        if host:
+            def dev(v, i=0):
+                return torch.as_tensor(np.ascontiguousarray(v.data[i * dof:(i + 1) * dof].reshape(-1)), dtype=tdt,
                                        device="cuda")
-            return d[i * dof:(i + 1) * dof].reshape(-1)
+        else:
+            def dev(v, i=0):
+                d = v.data
+                return d if i == 0 and d.is_contiguous() else d[i * dof:(i + 1) * dof].reshape(-1)
 
         um, uc, up = dev(solver_data.km1), dev(solver_data.k), dev(solver_data.kp1)
         psi = None
         if self.mesh.dim == 3:
             psi = dev(solver_data.k, 1 + self._aux_names.index("psi"))
         _, maps = self._device_sigmas()
-        out = torch.empty(dof, dtype=tdt, device="cuda")
+        out = torch.empty((dof, 1), dtype=tdt, device="cuda")
         sh = self.mesh.shape(include_bc=True, as_grid=True)
         if self.mesh.dim == 1:
             nx, ny, nz = 1, 1, sh[0]
@@ -383,7 +391,6 @@ class _CDATimeScalarCuda:
                                             self.mesh.dim, um.data_ptr(), uc.data_ptr(), up.data_ptr(),
                                             psi.data_ptr() if psi is not None else None, sx, sy, sz,
                                             nx, ny, nz, self.dt, out.data_ptr(), _native.stream_handle()))
-        out = out.reshape(-1, 1)
         return out.cpu().numpy() if host else out
 
     def _launch_step(self, f, vkm1, vk, out, C, rhs):
