@@ -160,16 +160,10 @@ struct Window {
 };
 
 // weights of the derivatives over the first differences e_j = v_{j+1} - v_j (FP64 path):
-// v'' = sum_j c_j (e_j - e_{-1-j}), v' = sum_j b_j (e_j + e_{-1-j}), j = 0..R-1, with
-// c_j = sum_{m>j} w2_m and b_j = sum_{m>j} w1_m
+// v'' = sum_j c_j (e_j - e_{-1-j}), j = 0..R-1, with c_j = sum_{m>j} w2_m
 __host__ __device__ constexpr double c2sum(int R, int j) {
     double s = 0;
     for (int m = j + 1; m <= R; ++m) s += d2w(R, m);
-    return s;
-}
-__host__ __device__ constexpr double c1sum(int R, int j) {
-    double s = 0;
-    for (int m = j + 1; m <= R; ++m) s += d1w(R, m);
     return s;
 }
 

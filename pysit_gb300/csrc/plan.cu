@@ -320,7 +320,7 @@ struct PlanT final : public pysit_plan {
     // ---- layout --------------------------------------------------------------
     int hx, hy, rows_y, ldz;
     long long fstride;  // elements per field per shot (256-byte multiple)
-    int bz, tx, ntz, ntx;
+    int tx;  // rows along x of a tile
     int nseg;
     std::vector<int> tasks2d;    // [ntasks][5] tiles of the 2D step: interior first, then shell
     int ntask2d[2] = {0, 0};     // tasks of each kind
@@ -489,32 +489,16 @@ struct PlanT final : public pysit_plan {
     }
 
     void choose_tiling() {
-        constexpr int V = V16<T>::N;
+        tx = 32;  // 1D has no tiles
         if (dim == 2) {
-            bz = kT2;
-            tx = tile_req ? tile_req : 32;
+            if (tile_req) tx = tile_req;
             strip2d = choose_strip2d();
             threads2d = choose_threads2d();
             build_tasks2d();
-            ntz = ntx = 1;
-            return;
-        }
-        if (dim == 3) {
+        } else if (dim == 3) {
             choose_tile3d();
             build_tasks3d();
-            ntz = ntx = 1;
-            return;
         }
-        // 1D: fewest loaded elements (tile + halo) per useful cell, bz >= 64
-        double best = 1e30;
-        for (int b : {64, 128, 256}) {
-            int tiles = (nz + b * V - 1) / (b * V);
-            double cost = (double)tiles * (b * V + 2 * kHalo) / nz;
-            if (cost < best - 1e-9) { best = cost; bz = b; }
-        }
-        tx = 32;
-        ntz = (nz + bz * V - 1) / (bz * V);
-        ntx = (nx + tx - 1) / tx;
     }
 
     // x-rows per thread of the 2D tiles.  More rows share more loads, but make fewer threads: a launch
@@ -1010,7 +994,7 @@ struct PlanT final : public pysit_plan {
     WaveParams<T> base_params(int g0, int gn) const {
         WaveParams<T> p{};
         p.nx = nx; p.ny = ny; p.nz = nz; p.ldz = ldz; p.rows_y = rows_y; p.fstride = fstride;
-        p.hx = hx; p.hy = hy; p.tx = tx; p.ty = 1; p.ntz = ntz; p.nty = 1; p.ntx = ntx; p.nshot = gn;
+        p.hx = hx; p.hy = hy; p.nshot = gn;
         p.c2 = at<T>(off.c2);
         p.sgx = at<T>(off.sgx); p.sgy = at<T>(off.sgy); p.sgz = at<T>(off.sgz);
         p.fcx = at<T>(off.fcx); p.fcy = at<T>(off.fcy); p.fcz = at<T>(off.fcz);
@@ -1099,9 +1083,9 @@ struct PlanT final : public pysit_plan {
             else if (mode == kRecomp) launch3d<RR, kRecomp>(p, s);             \
             else launch3d<RR, kAdj>(p, s);                                     \
         } else {                                                               \
-            if (mode == kFwd) launch_wave1d<T, RR, kFwd>(p, bz, s);            \
-            else if (mode == kRecomp) launch_wave1d<T, RR, kRecomp>(p, bz, s); \
-            else launch_wave1d<T, RR, kAdj>(p, bz, s);                         \
+            if (mode == kFwd) launch_wave1d<T, RR, kFwd>(p, s);            \
+            else if (mode == kRecomp) launch_wave1d<T, RR, kRecomp>(p, s); \
+            else launch_wave1d<T, RR, kAdj>(p, s);                         \
         }                                                                      \
     } while (0)
         switch (R) {

@@ -26,48 +26,6 @@ template <typename T> struct V16;
 template <> struct V16<float> { using type = float4; static constexpr int N = 4; };
 template <> struct V16<double> { using type = double2; static constexpr int N = 2; };
 
-template <typename T>
-struct alignas(16) VReg {
-    T v[V16<T>::N];
-};
-
-template <typename T>
-__device__ __forceinline__ VReg<T> vzero() {
-    VReg<T> r;
-#pragma unroll
-    for (int i = 0; i < V16<T>::N; ++i) r.v[i] = T(0);
-    return r;
-}
-template <typename T>
-__device__ __forceinline__ VReg<T> vld_ro(const T* p) {  // read-only path
-    VReg<T> r;
-    *reinterpret_cast<typename V16<T>::type*>(r.v) =
-        __ldg(reinterpret_cast<const typename V16<T>::type*>(p));
-    return r;
-}
-template <typename T>
-__device__ __forceinline__ VReg<T> vld(const T* p) {
-    VReg<T> r;
-    *reinterpret_cast<typename V16<T>::type*>(r.v) =
-        *reinterpret_cast<const typename V16<T>::type*>(p);
-    return r;
-}
-template <typename T>
-__device__ __forceinline__ VReg<T> vld_stream(const T* p) {  // read once: evict-first
-    VReg<T> r;
-    *reinterpret_cast<typename V16<T>::type*>(r.v) =
-        __ldcs(reinterpret_cast<const typename V16<T>::type*>(p));
-    return r;
-}
-template <typename T>
-__device__ __forceinline__ void vst(T* p, const VReg<T>& r) {
-    *reinterpret_cast<typename V16<T>::type*>(p) = *reinterpret_cast<const typename V16<T>::type*>(r.v);
-}
-template <typename T>
-__device__ __forceinline__ void vst_stream(T* p, const VReg<T>& r) {
-    __stcs(reinterpret_cast<typename V16<T>::type*>(p), *reinterpret_cast<const typename V16<T>::type*>(r.v));
-}
-
 // Kernel modes of the batched step.
 enum StepMode : int {
     kFwd = 0,     // forward step; records traces of u_k
@@ -111,10 +69,6 @@ struct WaveParams {
     int rows_y;              // ny + 2*HY
     long long fstride;       // elements between consecutive shots of one field
     int hx, hy;              // halos (4 / 0 in 2D)
-    // tiling
-    int tx;                  // rows swept per block along x
-    int ty;                  // 3D: y rows per block (blockDim.y)
-    int ntz, nty, ntx;       // tiles per shot along z, y, x
     int nshot;               // shots in this launch
     // wavefields (shot 0 base)
     T* u_prev;               // in: u_{k-1}; out: u_{k+1} (same cell, in place)
@@ -332,6 +286,6 @@ bool wave1d_sweeps(int nz, int npts);
 template <typename T, int R, int MODE>
 void launch_wave1d_sweep(const WaveParams<T>& p, Sweep1d<T> q, cudaStream_t s);
 template <typename T, int R, int MODE>
-void launch_wave1d(const WaveParams<T>& p, int bz, cudaStream_t s);
+void launch_wave1d(const WaveParams<T>& p, cudaStream_t s);
 
 }  // namespace pgb

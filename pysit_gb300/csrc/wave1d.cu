@@ -303,8 +303,7 @@ void launch_wave1d_sweep(const WaveParams<T>& p, Sweep1d<T> q, cudaStream_t s) {
 }
 
 template <typename T, int R, int MODE>
-void launch_wave1d(const WaveParams<T>& p, int bz, cudaStream_t s) {
-    (void)bz;
+void launch_wave1d(const WaveParams<T>& p, cudaStream_t s) {
     const int tb = 128;
     int ntile = ceil_div(p.nz, tb);
     int grid = ntile * p.nshot;
@@ -318,9 +317,9 @@ template bool wave1d_sweeps<double>(int, int);
     template void launch_wave1d_sweep<T, R, kFwd>(const WaveParams<T>&, Sweep1d<T>, cudaStream_t);    \
     template void launch_wave1d_sweep<T, R, kRecomp>(const WaveParams<T>&, Sweep1d<T>, cudaStream_t); \
     template void launch_wave1d_sweep<T, R, kAdj>(const WaveParams<T>&, Sweep1d<T>, cudaStream_t);    \
-    template void launch_wave1d<T, R, kFwd>(const WaveParams<T>&, int, cudaStream_t);    \
-    template void launch_wave1d<T, R, kRecomp>(const WaveParams<T>&, int, cudaStream_t); \
-    template void launch_wave1d<T, R, kAdj>(const WaveParams<T>&, int, cudaStream_t);
+    template void launch_wave1d<T, R, kFwd>(const WaveParams<T>&, cudaStream_t);    \
+    template void launch_wave1d<T, R, kRecomp>(const WaveParams<T>&, cudaStream_t); \
+    template void launch_wave1d<T, R, kAdj>(const WaveParams<T>&, cudaStream_t);
 PGB_INST1(float, 1)
 PGB_INST1(float, 2)
 PGB_INST1(float, 3)
