@@ -44,11 +44,11 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "FWI gradient shots/s, batched adjoint vs plain, 1\u00d7GB300 at \u22641e-3 rel err; Gcell/s"
-# DRAM bytes (read + write) per shot of a launch of each 2D step (interior + PML-shell kernels),
+# DRAM bytes (read + write) per shot of a launch of each 2D step (one kernel over all tiles),
 # from one ncu capture of the three step modes at 22 shots per launch
 # (profiles/wave2d_steps_cfg2_22shots_dram.md); a launch's traffic is this times its shots (the
 # kernels' traffic grows in proportion to the shots).
-TRAFFIC_PER_SHOT = {"forward": 174.3e6 / 22, "recompute": 198.5e6 / 22, "adjoint": 335.5e6 / 22}
+TRAFFIC_PER_SHOT = {"forward": 195.2e6 / 22, "recompute": 223.1e6 / 22, "adjoint": 345.1e6 / 22}
 
 
 def max_over_ranks(values, device):
@@ -425,7 +425,7 @@ def main():
     rn = float(plan.rnorm2.item())
 
     # ---- per-kernel roofline: each step kernel timed alone with CUDA events ------------
-    # (one launch = one 2D step of a shot group: interior + PML-shell kernels)
+    # (one launch = one 2D step of a shot group)
     # algorithmic bytes per cell: forward 4w interior / 8w PML; recompute +w (dWaveOp
     # out); adjoint +3w (dWaveOp in, imaging accumulator in and out)
     extra = {"forward": 0, "recompute": 1, "adjoint": 3}
@@ -498,7 +498,7 @@ def main():
                          "frac_distinct_note": "the same launch time against the bytes with C^2 read once per "
                                                "launch (it is shared by the launch's shots)",
                          "peak_kind": peak_kind,
-                         "kernel": f"2D {dom_name} step (interior + PML-shell kernels)",
+                         "kernel": f"2D {dom_name} step (wave2d_tile_kernel)",
                          "bytes_per_launch": dom["bytes_per_launch"], "launch_ms": dom["launch_ms"],
                          "modes": {k: {"launch_ms": v["launch_ms"], "achieved_gbs": v["achieved_gbs"],
                                        "frac": v["achieved_gbs"] / peak,

@@ -34,9 +34,9 @@
 //           per-column constants.
 // The arithmetic runs on cell pairs (packed f32x2 instructions in FP32).
 // Measured against the persistent warps with shared-memory row rings this kernel replaces
-// (us per step, before -> now): 1232 x 464 cells, order 8, FP32, 1 shot 33.9 -> 5.4, 16 shots
-// 61 -> 47, 64 shots forward / recompute / adjoint 181 / 185 / 224 -> 162 / 162 / 215;
-// 461 x 203, order 8, FP64, 6 shots 247 -> 77; 141 x 81, order 4, FP64, 1 shot 154 -> 7.8.
+// (us per step, before -> now): 1232 x 464 cells, order 8, FP32, 1 shot 33.9 -> 4.7, 16 shots
+// 61 -> 44, 64 shots forward / recompute / adjoint 181 / 185 / 224 -> 162 / 164 / 222;
+// 461 x 203, order 8, FP64, 6 shots 247 -> 60; 141 x 81, order 4, FP64, 1 shot 154 -> 5.5.
 // Staging the tiles in shared memory with bulk copies was slower or equal at every size (64
 // shots forward 159-178 us with four single-stage blocks per SM, 255-350 us with persistent
 // blocks, two stages and a copying warp).

@@ -19,14 +19,14 @@
 // the outputs through products of two or three sigmas, so the batched path
 // integrates it only where at least two axes are inside the padding.
 //
-// What bounds it: latency (long-scoreboard stalls with two 8-warp blocks per SM at 128 registers;
+// What bounds it: latency (long-scoreboard stalls with four 4-warp blocks per SM at 128 registers;
 // DRAM and L1 below 60 % busy).  Four planes per round need 13 vector loads of u_k per output
 // vector instead of 21, the faces' update 135-180 thread instructions per cell instead of the
 // general update's 276.  Measured against the kernels this one replaces, which walked 64 planes
 // one at a time in two kernels (us per step, before -> now): 440 x 440 x 340, order 8, FP32
-// forward / recompute / adjoint 593 / 595 / 707 -> 520 / 549 / 691; 121 x 107 x 95, order 4, FP32,
-// 4 shots 200 -> 95; 180 x 170 x 150, order 8, FP32 201 -> 69; 53 x 49 x 45, order 4, FP64, 2 shots
-// 708 -> 72.  Three blocks per SM (80 registers, spills) were 12 % slower.
+// forward / recompute / adjoint 593 / 595 / 707 -> 502 / 540 / 684; 121 x 107 x 95, order 4, FP32,
+// 4 shots 200 -> 80; 180 x 170 x 150, order 8, FP32 201 -> 57; 53 x 49 x 45, order 4, FP64, 2 shots
+// 708 -> 49.  Three blocks per SM (80 registers, spills) were 12 % slower.
 #pragma once
 #include "pairs.cuh"
 #include "tma.cuh"
