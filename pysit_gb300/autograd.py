@@ -88,7 +88,11 @@ def _make_function():
         def backward(ctx, gJ):
             C, grad_m = ctx.saved_tensors
             Cd = C.to(device=grad_m.device, dtype=torch.float64)
-            dC = grad_m * (-2.0 * ctx.dV) * Cd ** -3
+            # The general FP64 power took 7.7 ms of a 74 ms gradient on 400 x 400 x 300 cells.  The square of
+            # an FP32 (or narrower) C is exact in FP64, so the quotient rounds no more often than the power
+            # does; an FP64 C keeps the power (the quotient's error is 1.2 times as large there).
+            dC = grad_m * (-2.0 * ctx.dV)
+            dC = dC * Cd ** -3 if C.dtype == torch.float64 else dC / (Cd * Cd * Cd)
             return (gJ.to(dC.device) * dC).to(dtype=C.dtype, device=C.device), None
 
     return MisfitFunction
