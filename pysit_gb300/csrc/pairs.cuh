@@ -87,8 +87,7 @@ __device__ __forceinline__ void ldp(Pairs<float, 2>& r, const float* q) {
 }
 __device__ __forceinline__ void ldp(Pairs<float, 1>& r, const float* q) { r.p[0] = *reinterpret_cast<const unsigned long long*>(q); }
 __device__ __forceinline__ void ldp(Pairs<double, 1>& r, const double* q) { r.p[0] = *reinterpret_cast<const double2*>(q); }
-// the same through the read-only path: fields that the launch does not write, so that the compiler
-// may move these loads ahead of the stores of earlier rows
+// the same through the read-only path: C^2 and m1, which no step kernel writes (see pdl_handover)
 __device__ __forceinline__ void ldr(Pairs<float, 2>& r, const float* q) {
     const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2*>(q));
     r.p[0] = v.x; r.p[1] = v.y;
@@ -132,7 +131,7 @@ struct Window {
         for (int j = 0; j <= 2 * NB; ++j) {
             Pairs<T, NP> a;
             if (j == NB && centre) a = *centre;
-            else ldr(a, q + j * 2 * NP);
+            else ldp(a, q + j * 2 * NP);
 #pragma unroll
             for (int k = 0; k < NP; ++k) e[j * NP + k] = a.p[k];
         }

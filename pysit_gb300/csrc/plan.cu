@@ -1454,6 +1454,8 @@ struct PlanT final : public pysit_plan {
         WaveParams<T> p = base_params(0, gn);
         State st = mode == kAdj ? make_state(off.A, off.AX, off.AY, off.AZ, off.AS)
                                 : make_state(off.U, off.PX, off.PY, off.PZ, off.PS);
+        // adjoint steps read amplitudes ahead of their wait: not while earlier steps still record them
+        if (mode == kAdj) cudaMemsetAsync(ws + off.partial, 0, sizeof(double), s);
         for (int i = 0; i < n; ++i) {
             const int k = i % nsteps;
             bind_state(p, st);

@@ -118,7 +118,12 @@ __device__ __forceinline__ T one_sigma_fac(int dim, T dt, T dt2, T s) {
 // kernel before it to be complete, its writes visible, before it reads a wavefield, and then lets
 // the next one start (its blocks take the slots that the running one leaves and wait in turn: the
 // launch latency and the reads ahead of the wait overlap the running kernel).  What no step kernel
-// writes (tables, sigmas, C^2, injection operators and amplitudes) may be read before the wait.
+// writes (tables, sigmas, C^2, m1, injection operators) may be read before the wait, and through the
+// read-only path; so may the amplitudes, since a memset or another kernel always stands between the
+// steps that record traces and the adjoint steps that read the residual in their place.  Every wavefield, Phi, psi, dWaveOp and image is written by a kernel
+// that may still run when this one starts: it is read after the wait and with ordinary loads, since
+// __ldg is defined only for data that stay constant as long as the grid lives (the compiler may move
+// it across the wait, and L1 need not drop its lines).
 // Letting the next kernel start before the wait stacked several launches on the SMs: 141 x 81 cells
 // in FP64 8.2 us a step instead of 7.1 without any overlap.
 __device__ __forceinline__ void pdl_handover() {
@@ -211,7 +216,7 @@ __device__ __forceinline__ void record_pass(const WaveParams<T>& p, long long pa
                 w[q] = in ? __ldg(p.rec.w + e + q * G) : T(0);
             }
 #pragma unroll
-            for (int q = 0; q < kTaps; ++q) v[q] = e + q * G < e1 ? __ldg(u + off[q]) : T(0);
+            for (int q = 0; q < kTaps; ++q) v[q] = e + q * G < e1 ? u[off[q]] : T(0);
 #pragma unroll
             for (int q = 0; q < kTaps; ++q)
                 if (e + q * G < e1) acc += w[q] * v[q];

@@ -34,8 +34,8 @@
 //           per-column constants.
 // The arithmetic runs on cell pairs (packed f32x2 instructions in FP32).
 // Measured against the persistent warps with shared-memory row rings this kernel replaces
-// (us per step, before -> now): 1232 x 464 cells, order 8, FP32, 1 shot 33.9 -> 4.7, 16 shots
-// 61 -> 44, 64 shots forward / recompute / adjoint 181 / 185 / 224 -> 162 / 164 / 222;
+// (us per step, before -> now): 1232 x 464 cells, order 8, FP32, 1 shot 33.9 -> 4.4, 16 shots
+// 61 -> 43, 64 shots forward / recompute / adjoint 181 / 185 / 224 -> 157 / 166 / 222;
 // 461 x 203, order 8, FP64, 6 shots 247 -> 60; 141 x 81, order 4, FP64, 1 shot 154 -> 5.5.
 // Staging the tiles in shared memory with bulk copies was slower or equal at every size (64
 // shots forward 159-178 us with four single-stage blocks per SM, 255-350 us with persistent
@@ -110,7 +110,7 @@ __device__ __forceinline__ void tile_update(const WaveParams<T>& p, const T* rhs
     // rows past the tile's last one are read too (the next rows of the field, or its halo:
     // clamped to the strip's last row that exists) and not used
 #pragma unroll
-    for (int j = 0; j < RS + 2 * R; ++j) ldr(cv[j], u + (long long)(min(j, rows - r0 + 2 * R - 1) - R) * ldz);
+    for (int j = 0; j < RS + 2 * R; ++j) ldp(cv[j], u + (long long)(min(j, rows - r0 + 2 * R - 1) - R) * ldz);
 #pragma unroll
     for (int r = 0; r < RS; ++r) {
         const long long d = (long long)min(r, rows - r0 - 1) * ldz;
@@ -120,7 +120,31 @@ __device__ __forceinline__ void tile_update(const WaveParams<T>& p, const T* rhs
     if (PML) {
 #pragma unroll
         for (int j = 0; j < RS + 2 * R; ++j)
-            ldr(px[j], p.phx_in + sh + o0 + (long long)(min(j, rows - r0 + 2 * R - 1) - R) * ldz);
+            ldp(px[j], p.phx_in + sh + o0 + (long long)(min(j, rows - r0 + 2 * R - 1) - R) * ldz);
+    }
+    // Row r's neighbours along z and imaging operands.  A thread of one or two rows reads them all before
+    // it stores the first (1232 x 464, FP32, one shot: 4.4 us a step, 4.7 row by row); one of four rows
+    // reads them row by row (64 shots: 157 us, 161 with the next row's ahead of the stores), and so does
+    // the FP64 adjoint step (461 x 203 x 40 shots: 369 us, 372 up front).
+    constexpr bool FRONT = RS < 4 && !(sizeof(T) == 8 && MODE == kAdj);
+    constexpr int NF = FRONT ? RS : 1;
+    Window<T, NP, NB> wf[NF], wpf[NF];
+    Pairs<T, NP> dwf[NF], icf[NF];
+    auto fetch = [&](int r) {
+        const int f = FRONT ? r : 0;
+        const long long o = o0 + (long long)r * ldz;
+        wf[f].load(u + (long long)r * ldz - HZ, &cv[R + r]);
+        if ((MODE == kAdj && img) || MODE == kBorn) {  // for kBorn: dWaveOp0 and m1
+            ldp(dwf[f], p.dw_in + sh + o);
+            if (MODE == kBorn) ldr(icf[f], p.m1 + o);
+            else ldp(icf[f], p.ic + sh + o);
+        }
+        if (PML) wpf[f].load(p.phz_in + sh + o - HZ, nullptr);
+    };
+    if (FRONT) {
+#pragma unroll
+        for (int r = 0; r < RS; ++r)
+            if (r0 + r < rows) fetch(r);
     }
     {
 #pragma unroll
@@ -128,21 +152,13 @@ __device__ __forceinline__ void tile_update(const WaveParams<T>& p, const T* rhs
             if (r0 + r >= rows) break;
             const int xr = x0 + r0 + r;
             const long long o = o0 + (long long)r * ldz;
-            Window<T, NP, NB> w, wp;
-            w.load(u + (long long)r * ldz - HZ, &cv[R + r]);
-            Pairs<T, NP> dwi, ici;
-            if ((MODE == kAdj && img) || MODE == kBorn) {  // for kBorn: dWaveOp0 and m1
-                ldr(dwi, p.dw_in + sh + o);
-                if (MODE == kBorn) ldr(ici, p.m1 + o);
-                else ldp(ici, p.ic + sh + o);
-            }
+            if (!FRONT) fetch(r);
+            const auto &w = wf[FRONT ? r : 0], &wp = wpf[FRONT ? r : 0];
+            const auto &dwi = dwf[FRONT ? r : 0], &ici = icf[FRONT ? r : 0];
             T sx = T(0), mgx = T(0);
-            if (PML) {
-                wp.load(p.phz_in + sh + o - HZ, nullptr);
-                if (KIND == 1) {
-                    sx = sxr[r];
-                    mgx = mxr[r];
-                }
+            if (KIND == 1) {
+                sx = sxr[r];
+                mgx = mxr[r];
             }
             T rh[V];
             const bool inj_row = injz && xr >= ib.x && xr < ib.y;

@@ -24,8 +24,8 @@
 // vector instead of 21, the faces' update 135-180 thread instructions per cell instead of the
 // general update's 276.  Measured against the kernels this one replaces, which walked 64 planes
 // one at a time in two kernels (us per step, before -> now): 440 x 440 x 340, order 8, FP32
-// forward / recompute / adjoint 593 / 595 / 707 -> 502 / 540 / 684; 121 x 107 x 95, order 4, FP32,
-// 4 shots 200 -> 80; 180 x 170 x 150, order 8, FP32 201 -> 57; 53 x 49 x 45, order 4, FP64, 2 shots
+// forward / recompute / adjoint 593 / 595 / 707 -> 491 / 551 / 671; 121 x 107 x 95, order 4, FP32,
+// 4 shots 200 -> 80; 180 x 170 x 150, order 8, FP32 201 -> 56; 53 x 49 x 45, order 4, FP64, 2 shots
 // 708 -> 49.  Three blocks per SM (80 registers, spills) were 12 % slower.
 #pragma once
 #include "pairs.cuh"
@@ -40,10 +40,6 @@ template <> struct Vec3<double> { using type = double2; static constexpr int N =
 
 template <typename T>
 __device__ __forceinline__ typename Vec3<T>::type ldv(const T* q) {
-    return __ldg(reinterpret_cast<const typename Vec3<T>::type*>(q));
-}
-template <typename T>
-__device__ __forceinline__ typename Vec3<T>::type ldv_plain(const T* q) {
     return *reinterpret_cast<const typename Vec3<T>::type*>(q);
 }
 
@@ -269,8 +265,8 @@ __device__ __forceinline__ void general_update(const WaveParams<T>& p, const T* 
 #pragma unroll
             for (int v = 0; v < V; ++v) ps[v] = T(0);
         }
-        const VT uo_v = ldv_plain(p.u_prev + sh + o);
-        const VT c2_v = ldv(p.c2 + o);
+        const VT uo_v = ldv(p.u_prev + sh + o);
+        const VT c2_v = __ldg(reinterpret_cast<const VT*>(p.c2 + o));
         alignas(16) T un[V];
         if (sx != T(0) || sy != T(0) || any_sz) {
             // psi derivatives where two sigmas meet (zero elsewhere, as the products they enter)
@@ -364,7 +360,7 @@ __device__ __forceinline__ void general_update(const WaveParams<T>& p, const T* 
         }
         if (MODE == kAdj && p.image) {
             const VT dw_v = __ldcs(reinterpret_cast<const VT*>(p.dw_in + sh + o));
-            const VT ic_v = ldv_plain(p.ic + sh + o);
+            const VT ic_v = ldv(p.ic + sh + o);
             alignas(16) T ico[V];
 #pragma unroll
             for (int v = 0; v < V; ++v) ico[v] = vc<T>(ic_v, v) + uc[v] * vc<T>(dw_v, v);
@@ -436,17 +432,11 @@ __device__ __forceinline__ void interior_planes(const WaveParams<T>& p, const T*
     const long long ys = p.ldz, xs = (long long)p.rows_y * p.ldz;
     const T* u = p.u_cur + sh + o0;
     P Fx[RX][NP];
-    // what the planes' stores write is read before the first of them
-    Pairs<T, NP> um[RX];
-#pragma unroll
-    for (int r = 0; r < RX; ++r) {
-        ldp(um[r], p.u_prev + sh + o0 + (long long)min(r, n - 1) * xs);
-    }
     {
         Pairs<T, NP> cv[RX + 2 * R];
         // planes past the tile's last one are read too (the next planes or the halo) and not used
 #pragma unroll
-        for (int q = 0; q < RX + 2 * R; ++q) ldr(cv[q], u + (long long)(min(q, n - 1 + 2 * R) - R) * xs);
+        for (int q = 0; q < RX + 2 * R; ++q) ldp(cv[q], u + (long long)(min(q, n - 1 + 2 * R) - R) * xs);
 #pragma unroll
         for (int r = 0; r < RX; ++r)
 #pragma unroll
@@ -465,24 +455,35 @@ __device__ __forceinline__ void interior_planes(const WaveParams<T>& p, const T*
                 Fx[r][k] = F;
             }
     }
+    // The other operands of plane r.  The adjoint step reads them before plane r - 1 is stored (440 x
+    // 440 x 340, order 8, FP32: 671 us, 694 after its stores); the other modes, which hold fewer
+    // operands a plane, after (forward 491 us, 498 before).
+    constexpr bool AHEAD = MODE == kAdj;
+    Window<T, NP, NB> w;
+    Pairs<T, NP> ya[2 * R], cc, um, dwi, ici;
+    auto fetch = [&](int r) {
+        const long long o = o0 + (long long)r * xs;
+        const T* ur = u + (long long)r * xs;
+        w.load(ur - HZ, nullptr);
+#pragma unroll
+        for (int m = 1; m <= R; ++m) {
+            ldp(ya[R - m], ur - m * ys);
+            ldp(ya[R + m - 1], ur + m * ys);
+        }
+        ldr(cc, p.c2 + o);
+        ldp(um, p.u_prev + sh + o);
+        if (MODE == kAdj && p.image) {
+            ldp(dwi, p.dw_in + sh + o);
+            ldp(ici, p.ic + sh + o);
+        }
+    };
+    if (AHEAD) fetch(0);
 #pragma unroll
     for (int r = 0; r < RX; ++r) {
         if (r >= n) break;
         const long long o = o0 + (long long)r * xs;
-        const T* ur = u + (long long)r * xs;
-        Window<T, NP, NB> w;
-        w.load(ur - HZ, nullptr);
-        Pairs<T, NP> ya[2 * R], cc, dwi, ici, un, dwo, ico;
-#pragma unroll
-        for (int m = 1; m <= R; ++m) {
-            ldr(ya[R - m], ur - m * ys);
-            ldr(ya[R + m - 1], ur + m * ys);
-        }
-        ldr(cc, p.c2 + o);
-        if (MODE == kAdj && p.image) {
-            ldr(dwi, p.dw_in + sh + o);
-            ldp(ici, p.ic + sh + o);
-        }
+        if (!AHEAD) fetch(r);
+        Pairs<T, NP> un, dwo, ico;
         const bool inj_row = inj_col && x + r >= ib.x0 && x + r < ib.x1;
 #pragma unroll
         for (int k = 0; k < NP; ++k) {
@@ -509,7 +510,7 @@ __device__ __forceinline__ void interior_planes(const WaveParams<T>& p, const T*
                 rh[1] = ib.at(rhs, x + r, j, zl + 2 * k + 1);
                 if (MODE != kAdj) F = O::add(F, O::mk(rh[0], rh[1]));
             }
-            const P uo = um[r].p[k], c2 = cc.p[k];
+            const P uo = um.p[k], c2 = cc.p[k];
             // u_{k+1} = dt^2 C^2 F - (u_{k-1} - 2 u_k)
             const P q = O::fma(O::dup(T(-2)), uc, uo);
             un.p[k] = O::fma(O::mul(O::dup(p.dt2), c2), F, O::mul(q, O::dup(T(-1))));
@@ -519,6 +520,7 @@ __device__ __forceinline__ void interior_planes(const WaveParams<T>& p, const T*
             if (MODE == kAdj) ico.p[k] = O::fma(uc, dwi.p[k], ici.p[k]);
             if (MODE == kFwd || (MODE == kRecomp && p.nan_check)) chk.see(un.p[k]);
         }
+        if (AHEAD && r + 1 < RX && r + 1 < n) fetch(r + 1);
         stp(p.u_prev + sh + o, un);
         if (MODE == kRecomp && p.dw_out) stp_cs(p.dw_out + sh + o, dwo);
         if (MODE == kAdj && p.image) stp(p.ic + sh + o, ico);
@@ -551,16 +553,10 @@ __device__ __forceinline__ void face_planes(const WaveParams<T>& p, const T* rhs
     const long long ys = p.ldz, xs = (long long)p.rows_y * p.ldz;
     const T* u = p.u_cur + sh + o0;
     P Fx[RX][NP], dux[RX][NP], dpx[RX][NP];
-    // what the planes' stores write is read before the first of them
-    Pairs<T, NP> umr[RX];
-#pragma unroll
-    for (int r = 0; r < RX; ++r) {
-        ldp(umr[r], p.u_prev + sh + o0 + (long long)min(r, n - 1) * xs);
-    }
     {
         Pairs<T, NP> cv[RX + 2 * R];
 #pragma unroll
-        for (int q = 0; q < RX + 2 * R; ++q) ldr(cv[q], u + (long long)(min(q, n - 1 + 2 * R) - R) * xs);
+        for (int q = 0; q < RX + 2 * R; ++q) ldp(cv[q], u + (long long)(min(q, n - 1 + 2 * R) - R) * xs);
 #pragma unroll
         for (int r = 0; r < RX; ++r)
 #pragma unroll
@@ -576,7 +572,7 @@ __device__ __forceinline__ void face_planes(const WaveParams<T>& p, const T* rhs
     if (needx) {
         Pairs<T, NP> px[RX + 2 * R];
 #pragma unroll
-        for (int q = 0; q < RX + 2 * R; ++q) ldr(px[q], p.phx_in + sh + o0 + (long long)(min(q, n - 1 + 2 * R) - R) * xs);
+        for (int q = 0; q < RX + 2 * R; ++q) ldp(px[q], p.phx_in + sh + o0 + (long long)(min(q, n - 1 + 2 * R) - R) * xs);
 #pragma unroll
         for (int r = 0; r < RX; ++r)
 #pragma unroll
@@ -592,19 +588,21 @@ __device__ __forceinline__ void face_planes(const WaveParams<T>& p, const T* rhs
         if (r >= n) break;
         const int i = x + r;
         const long long o = o0 + (long long)r * xs;
-        const T* ur = u + (long long)r * xs;
         const T sx = AX == 0 ? __ldg(p.sgx + i) : T(0);
         const bool pxin = AX == 0 && (i < p.pxl || i >= p.nx - p.pxr);
+        const T* ur = u + (long long)r * xs;
+        Window<T, NP, NB> w;
+        w.load(ur - HZ, nullptr);
+        Pairs<T, NP> ya[2 * R], cc, um;
+#pragma unroll
+        for (int m = 1; m <= R; ++m) {
+            ldp(ya[R - m], ur - m * ys);
+            ldp(ya[R + m - 1], ur + m * ys);
+        }
+        ldr(cc, p.c2 + o);
+        ldp(um, p.u_prev + sh + o);
         P F[NP], duy[NP], duz[NP], uc[NP];
         {
-            Window<T, NP, NB> w;
-            w.load(ur - HZ, nullptr);
-            Pairs<T, NP> ya[2 * R];
-#pragma unroll
-            for (int m = 1; m <= R; ++m) {
-                ldr(ya[R - m], ur - m * ys);
-                ldr(ya[R + m - 1], ur + m * ys);
-            }
 #pragma unroll
             for (int k = 0; k < NP; ++k) {
                 const int c = C0 + 2 * k;
@@ -634,8 +632,8 @@ __device__ __forceinline__ void face_planes(const WaveParams<T>& p, const T* rhs
             Pairs<T, NP> t[2 * R];
 #pragma unroll
             for (int m = 1; m <= R; ++m) {
-                ldr(t[R - m], p.phy_in + sh + o - m * ys);
-                ldr(t[R + m - 1], p.phy_in + sh + o + m * ys);
+                ldp(t[R - m], p.phy_in + sh + o - m * ys);
+                ldp(t[R + m - 1], p.phy_in + sh + o + m * ys);
             }
 #pragma unroll
             for (int k = 0; k < NP; ++k) {
@@ -665,9 +663,7 @@ __device__ __forceinline__ void face_planes(const WaveParams<T>& p, const T* rhs
 #pragma unroll
                 for (int k = 0; k < NP; ++k) F[k] = O::add(F[k], O::mk(rh[2 * k], rh[2 * k + 1]));
         }
-        Pairs<T, NP> cc, un, dwo;
-        const Pairs<T, NP>& um = umr[r];
-        ldr(cc, p.c2 + o);
+        Pairs<T, NP> un, dwo, nx_, ny_, nz_, dwi, ici;
         const T s1 = AX == 0 ? sx : col.sy;  // the face's sigma where it is the same for the vector
         const bool pml = AX == 2 ? col.any_sz : s1 != T(0);
         const bool ring = !(col.zall && i > 0 && i < p.nx - 1);
@@ -684,9 +680,9 @@ __device__ __forceinline__ void face_planes(const WaveParams<T>& p, const T* rhs
             un.p[k] = plain[k];
         }
         if (pml) {
-            Pairs<T, NP> phx, phy, phz, nx_, ny_, nz_;
-            ldr(phx, p.phx_in + sh + o);
-            ldr(phy, p.phy_in + sh + o);
+            Pairs<T, NP> phx, phy, phz;
+            ldp(phx, p.phx_in + sh + o);
+            ldp(phy, p.phy_in + sh + o);
             const T f1 = AX == 0 ? __ldg(p.fcx + i) : AX == 1 ? __ldg(p.fcy + j) : T(0);
 #pragma unroll
             for (int k = 0; k < NP; ++k) {
@@ -717,9 +713,6 @@ __device__ __forceinline__ void face_planes(const WaveParams<T>& p, const T* rhs
                     nz_.p[k] = mask(nz_.p[k], k);
                 }
             }
-            stp(p.phx_out + sh + o, nx_);
-            stp(p.phy_out + sh + o, ny_);
-            stp(p.phz_out + sh + o, nz_);
         }
         if (ring)
 #pragma unroll
@@ -738,7 +731,6 @@ __device__ __forceinline__ void face_planes(const WaveParams<T>& p, const T* rhs
                 un.p[k] = O::mk(t[0], t[1]);
             }
         }
-        stp(p.u_prev + sh + o, un);
         if (MODE == kRecomp && p.dw_out) {
             // dWaveOp = C^2 F + (sm - s)(u' - u_{k-1})/(2dt)
             const T m1 = AX == 0 ? __ldg(p.mgx + i) : col.my;
@@ -750,16 +742,21 @@ __device__ __forceinline__ void face_planes(const WaveParams<T>& p, const T* rhs
                                    O::mul(O::mul(O::sub(M, S), O::sub(un.p[k], um.p[k])), O::dup(p.i2dt)));
                 dwo.p[k] = ring ? mask(d, k) : d;
             }
-            stp_cs(p.dw_out + sh + o, dwo);
         }
         if (MODE == kAdj && p.image) {
-            Pairs<T, NP> dwi, ici;
+            ldp(dwi, p.dw_in + sh + o);
             ldp(ici, p.ic + sh + o);
-            ldr(dwi, p.dw_in + sh + o);
 #pragma unroll
             for (int k = 0; k < NP; ++k) ici.p[k] = O::fma(uc[k], dwi.p[k], ici.p[k]);
-            stp(p.ic + sh + o, ici);
         }
+        if (pml) {
+            stp(p.phx_out + sh + o, nx_);
+            stp(p.phy_out + sh + o, ny_);
+            stp(p.phz_out + sh + o, nz_);
+        }
+        stp(p.u_prev + sh + o, un);
+        if (MODE == kRecomp && p.dw_out) stp_cs(p.dw_out + sh + o, dwo);
+        if (MODE == kAdj && p.image) stp(p.ic + sh + o, ici);
         if (MODE == kFwd || (MODE == kRecomp && p.nan_check))
 #pragma unroll
             for (int k = 0; k < NP; ++k) chk.see(un.p[k]);
