@@ -1,0 +1,67 @@
+"""The order of a plan's copies, launches, events and waits, read on any host from a stand-in for the
+CUDA runtime (fake_cudart.cpp, preloaded into a child process): no device, no kernel runs."""
+import os
+import shutil
+import subprocess
+import sys
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+
+CHILD = """
+import ctypes as C, sys
+import numpy as np
+sys.path[:0] = [%r, %r]
+from pysit_gb300 import _native
+from test_task_tables import _desc
+lib = _native.load()
+fake = C.CDLL(None)
+fake.fake_log.restype = C.c_char_p
+keep = []
+def plan(d):
+    h, n = C.c_void_p(), C.c_uint64()
+    _native.check(lib.pysit_plan_create(C.byref(d), C.byref(h)))
+    _native.check(lib.pysit_plan_workspace_bytes(h, C.byref(n)))
+    raw = np.empty(n.value + 256, np.uint8)
+    keep.append(raw)
+    p = (raw.ctypes.data + 255) // 256 * 256
+    _native.check(lib.pysit_plan_bind_workspace(h, C.c_void_p(p), n, C.c_void_p(7)))
+    return h
+def model(h, d):
+    c = np.full(d.n[0] * d.n[1] * d.n[2], 2000.0)
+    keep.append(c)
+    _native.check(lib.pysit_plan_set_model(h, C.c_void_p(c.ctypes.data), C.c_void_p(7)))
+def log():
+    return fake.fake_log().decode().splitlines()
+""" % (ROOT, HERE)
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    from pysit_gb300 import build
+    build.build()
+    so = str(tmp_path_factory.mktemp("fake") / "fake_cudart.so")
+    inc = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(build._nvcc()))), "include")
+    subprocess.run([shutil.which("g++"), "-shared", "-fPIC", "-std=c++17", "-I", inc,
+                    os.path.join(HERE, "fake_cudart.cpp"), "-o", so], check=True)
+    return so
+
+
+def _run(fake, code, **env):
+    r = subprocess.run([sys.executable, "-c", CHILD + code], capture_output=True, text=True,
+                       env={**os.environ, "LD_PRELOAD": fake, **env})
+    assert r.returncode == 0, r.stderr
+    return r.stdout.splitlines()
+
+
+@pytest.mark.parametrize("dim,n", [(1, (1, 1, 120)), (2, (40, 1, 36)), (3, (20, 18, 24))])
+def test_bind_returns_with_the_workspace_complete(fake, dim, n):
+    """Everything that bind enqueues is waited for before it returns, so that another stream may
+    use the plan next."""
+    out = _run(fake, f"d = _desc(keep, {dim}, {n}, ((4, 4),) * 3, 4, _native.PYSIT_F64)\n"
+                     "plan(d)\nprint('\\n'.join(log()))")
+    work = [i for i, l in enumerate(out) if l.split()[0] in ("launch", "memcpy", "memset")]
+    assert any("one_sigma" in out[i] for i in work)
+    assert "sync 7" in out[work[-1] + 1:]
