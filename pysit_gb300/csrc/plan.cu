@@ -941,14 +941,15 @@ struct PlanT final : public pysit_plan {
         if ((rc = upload(off.recw, tmp = toT(rec_ws), s))) return rc;
         if ((rc = dim == 3 ? upload(off.tasks, tiles3d, s) : upload(off.tasks, tiles2d, s))) return rc;
         if ((rc = upload(off.shsteps, shot_steps, s))) return rc;
-        PGB_CHECK_CUDA(cudaStreamSynchronize(s));
-        if (!cap) PGB_CHECK_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
         auto one_sigma = [&](size_t sigma, size_t out, int n) {
             one_sigma_kernel<T><<<grid_for(n, 256), 256, 0, s>>>(at<T>(sigma), n, dim, T(dt), T(dt * dt), at<T>(out));
         };
         one_sigma(off.sgx, off.fcx, nx);
         one_sigma(off.sgy, off.fcy, ny);
         one_sigma(off.sgz, off.fcz, nz);
+        PGB_CHECK_CUDA(cudaGetLastError());
+        PGB_CHECK_CUDA(cudaStreamSynchronize(s));  // the workspace is complete: any stream may run the plan
+        if (!cap) PGB_CHECK_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
         if (overlap) {
             if (!aux) PGB_CHECK_CUDA(cudaStreamCreateWithFlags(&aux, cudaStreamNonBlocking));
             for (auto e : {&ev_fork, &ev_ready[0], &ev_ready[1], &ev_free[0], &ev_free[1]})
