@@ -11,12 +11,12 @@
 //
 // One thread per cell, z (the contiguous axis) on threadIdx.x.  Taps outside
 // [0, n) are zero, which is the zero extension of the reference.  In FP64 the FP64 units
-// bound the step (86% busy; DRAM 7%), so what counts is FP64 instructions per cell: first-
-// derivative taps carry 1/h, zeros are tested on the integer units, first derivatives
-// are taken only where they enter, and the PML update is one quotient,
+// bound the step (86% busy; DRAM 7%), so what counts is FP64 instructions per cell: zeros are
+// tested on the integer units, first derivatives are taken only where they enter, and the PML
+// update is one quotient,
 //     u' = 2 u - u_{k-1} + (2 dt^2 C^2 (F - ...) + 2 dt s (u_{k-1} - u) - 2 dt^2 s2 u) / (2 + dt s),
 // in place of three; only a small correction is divided, so the last sum sets the rounding.
-// Measured, one time_step + compute_dWaveOp on 193 x 193 x 153 cells, order 4, FP64: 1266 -> 788 us.
+// Measured, one time_step + compute_dWaveOp on 193 x 193 x 153 cells, order 4, FP64: 1266 -> 801 us.
 #include <algorithm>
 
 #include "common.cuh"
@@ -45,10 +45,10 @@ __device__ __forceinline__ bool nonfinite(double a) {
     return ((unsigned)__double2hiint(a) & 0x7ff00000u) == 0x7ff00000u;
 }
 
-// one axis: first-derivative taps over h for m = 1..R, and 1 / h^2
+// one axis: 1 / h and 1 / h^2
 template <typename T>
 struct Axis {
-    T c1[4], id2;
+    T id, id2;
 };
 
 // the 2R+1 values of v along one axis around position p of n, element stride s
@@ -60,22 +60,27 @@ struct Taps {
         for (int m = -R; m <= R; ++m) t[m + R] = p + m < 0 || p + m >= n ? T(0) : __ldg(v + idx + m * s);
     }
     // acc + second derivative.  The taps stay unscaled and each axis cancels by itself: with 1/h^2
-    // in the taps and the centre taps of all axes taken at once (709 us instead of 788) the FP64
-    // rounding error of u' in plain cells was 1.4 to 2 times as large.
+    // in the taps and the centre taps of all axes taken at once (709 us instead of 801) the FP64
+    // rounding error of u' in plain cells was 1.4 to 2 times as large.  Fused multiply-adds by name:
+    // left to the compiler, the product of u and the centre weight was taken once, rounded, for the
+    // three axes (error of u' in plain cells 1.06 to 1.15 times as large).
     __device__ __forceinline__ T add_d2(T acc, const Axis<T>& x) const {
         T b = 0;
 #pragma unroll
-        for (int m = -R; m <= R; ++m) b += T(d2tap(R, m)) * t[m + R];
-        return acc + b * x.id2;
+        for (int m = -R; m <= R; ++m) b = ::fma(T(d2tap(R, m)), t[m + R], b);
+        return ::fma(b, x.id2, acc);
     }
-    __device__ __forceinline__ T add_d1(T acc, const Axis<T>& x) const {
+    // First derivative from the differences of opposite taps, 1/h last.  1/h in the taps saves that
+    // multiplication, but rounds each tap twice: error of Phi' at orders 6 and 8 1.05 to 1.3 times that
+    // of the taps summed one by one (spacings 7.3 to 12.5); this form 0.90 to 0.97 times.
+    __device__ __forceinline__ T sum_d1() const {
+        T b = 0;
 #pragma unroll
-        for (int m = 1; m <= R; ++m) acc += x.c1[m - 1] * t[R + m];
-#pragma unroll
-        for (int m = 1; m <= R; ++m) acc -= x.c1[m - 1] * t[R - m];
-        return acc;
+        for (int m = R; m >= 1; --m) b = ::fma(T(d1w(R, m)), t[R + m] - t[R - m], b);
+        return b;
     }
-    __device__ __forceinline__ T d1(const Axis<T>& x) const { return add_d1(T(0), x); }
+    __device__ __forceinline__ T add_d1(T acc, const Axis<T>& x) const { return ::fma(sum_d1(), x.id, acc); }
+    __device__ __forceinline__ T d1(const Axis<T>& x) const { return sum_d1() * x.id; }
     // a tap beside the centre is nonzero
     __device__ __forceinline__ bool any_nonzero() const {
         bool any = false;
@@ -93,6 +98,12 @@ struct Taps {
         return any;
     }
 };
+
+// u_{k+1} = dt^2 A - (u_{k-1} - 2 u_k), A = C^2 F: the product is added last, in one rounding
+template <typename T>
+__device__ __forceinline__ T plain_update(T A, T um, T uc, T dt2) {
+    return ::fma(dt2, A, ::fma(T(2), uc, -um));
+}
 
 // u_{k+1} where a sigma is nonzero: A = C^2 (F - ...), a = dt * sum of the sigmas; w = the sum of
 // their products times 2 dt^2, zero where only one is nonzero
@@ -135,7 +146,7 @@ __global__ void __launch_bounds__(256) step1d_kernel(Step1DArgs<T> a) {
         a.kp1_u[k] = pml_update(A, um, uc, az, T(0), a.dt2x2);
     } else {
         a.kp1_phiz[k] = ph;
-        a.kp1_u[k] = a.dt2 * A - (um - T(2) * uc);
+        a.kp1_u[k] = plain_update(A, um, uc, a.dt2);
     }
 }
 
@@ -177,7 +188,7 @@ __global__ void __launch_bounds__(256) step2d_kernel(Step2DArgs<T> a) {
     } else {
         a.kp1_phix[idx] = phx;
         a.kp1_phiz[idx] = phz;
-        a.kp1_u[idx] = a.dt2 * A - (um - T(2) * uc);
+        a.kp1_u[idx] = plain_update(A, um, uc, a.dt2);
     }
 }
 
@@ -250,7 +261,7 @@ __global__ void __launch_bounds__(128, step3d_blocks(R)) step3d_kernel(Step3DArg
         a.kp1_phix[idx] = a.k_phix[idx];
         a.kp1_phiy[idx] = a.k_phiy[idx];
         a.kp1_phiz[idx] = a.k_phiz[idx];
-        a.kp1_u[idx] = a.dt2 * (c2 * F) - (um - T(2) * uc);
+        a.kp1_u[idx] = plain_update(c2 * F, um, uc, a.dt2);
     }
 }
 
@@ -294,20 +305,15 @@ Prof<T> prof(const void* l, int nl, const void* r, int nr) {
 }
 
 template <typename T>
-Axis<T> axis(int order, double h) {
-    Axis<T> x{};
-    const int R = order / 2;
-    const T id = T(1.0 / h);
-    x.id2 = T(1.0 / (T(h) * T(h)));
-    for (int m = 1; m <= R; ++m) x.c1[m - 1] = T(d1tap(R, m)) * id;
-    return x;
+Axis<T> axis(double h) {
+    return Axis<T>{T(1.0 / h), T(1.0 / (T(h) * T(h)))};
 }
 
 template <typename T>
 int launch1d(int order, const void* km1_u, const void* k_phiz, const void* k_u, const void* C,
              const void* rhs, const void* zl, int nzl, const void* zr, int nzr, double dt,
              double dz, int nz, void* kp1_phiz, void* kp1_u, cudaStream_t s) {
-    const Axis<T> z = axis<T>(order, dz);
+    const Axis<T> z = axis<T>(dz);
     Step1DArgs<T> a{(const T*)km1_u, (const T*)k_phiz, (const T*)k_u, (const T*)C, (const T*)rhs,
                     prof<T>(zl, nzl, zr, nzr), z, T(dt), T(T(dt) * T(dt)), T(2) * T(T(dt) * T(dt)),
  nz, (T*)kp1_phiz, (T*)kp1_u};
@@ -328,7 +334,7 @@ int launch2d(int order, const void* km1_u, const void* k_phix, const void* k_phi
              const void* xr, int nxr, const void* zl, int nzl, const void* zr, int nzr,
              double dt, double dx, double dz, int nx, int nz, void* kp1_phix, void* kp1_phiz,
              void* kp1_u, cudaStream_t s) {
-    const Axis<T> x = axis<T>(order, dx), z = axis<T>(order, dz);
+    const Axis<T> x = axis<T>(dx), z = axis<T>(dz);
     Step2DArgs<T> a{(const T*)km1_u, (const T*)k_phix, (const T*)k_phiz, (const T*)k_u,
                     (const T*)C, (const T*)rhs, prof<T>(xl, nxl, xr, nxr), prof<T>(zl, nzl, zr, nzr),
                     x, z, T(dt), T(T(dt) * T(dt)), T(2) * T(T(dt) * T(dt)), nx, nz, (T*)kp1_phix, (T*)kp1_phiz, (T*)kp1_u};
@@ -350,7 +356,7 @@ int launch3d(int order, const void* km1_u, const void* k_phix, const void* k_phi
              int nyl, const void* yr, int nyr, const void* zl, int nzl, const void* zr, int nzr,
              double dt, double dx, double dy, double dz, int nx, int ny, int nz, void* kp1_phix,
              void* kp1_phiy, void* kp1_phiz, void* kp1_psi, void* kp1_u, cudaStream_t s) {
-    const Axis<T> x = axis<T>(order, dx), y = axis<T>(order, dy), z = axis<T>(order, dz);
+    const Axis<T> x = axis<T>(dx), y = axis<T>(dy), z = axis<T>(dz);
     Step3DArgs<T> a{(const T*)km1_u, (const T*)k_phix, (const T*)k_phiy, (const T*)k_phiz,
                     (const T*)k_psi, (const T*)k_u, (const T*)C, (const T*)rhs,
                     prof<T>(xl, nxl, xr, nxr), prof<T>(yl, nyl, yr, nyr), prof<T>(zl, nzl, zr, nzr),
