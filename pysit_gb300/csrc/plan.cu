@@ -312,7 +312,7 @@ struct PlanT final : public pysit_plan {
     unsigned wait_polls = 0;     // tests of the wait that wait_fault adds (pysit_plan_desc.wait_polls)
     int wait_fault = 0;          // test aid: a wait of the 2D step kernels runs out (pysit_plan_desc.wait_fault)
     std::vector<int> shot_steps; // record length of each shot in steps (empty: all nsteps)
-    size_t task_cap = 0;         // ints the task buffer holds (enough for any tile the tuner may set)
+    size_t task_cap = 0;         // tiles the task buffer holds (enough for any that the tuner may set)
     double dx, dy, dz, dt;
     int pad_lo[3], pad_hi[3];
     int pl[3], pr[3];  // PML-state widths (kernel profile lengths)
@@ -565,6 +565,10 @@ struct PlanT final : public pysit_plan {
         const int rows = std::min(once, tx);
         const int nxc = (xb - xa + rows - 1) / rows;
         const int wx = std::min(rows, ((xb - xa + nxc - 1) / nxc + strip2d - 1) / strip2d * strip2d);
+        if (counting) {
+            counted += zs.size() * ((xb - xa + wx - 1) / wx);
+            return;
+        }
         for (int x = xa; x < xb; x += wx)
             for (auto& z : zs) {
                 int t[5] = {x, std::min(xb, x + wx), z.first, z.second, kind};
@@ -573,7 +577,7 @@ struct PlanT final : public pysit_plan {
     }
     void build_tasks2d() {
         tasks2d.clear();
-        build_tasks2d_();
+        draw_tasks2d();
         // interior tasks were added first
         ntask2d[0] = ntask2d[1] = 0;
         for (size_t t = 0; t < tasks2d.size(); t += 5) ++ntask2d[tasks2d[t + 4] ? 1 : 0];
@@ -605,7 +609,7 @@ struct PlanT final : public pysit_plan {
                                kind && xoff ? 2 : kind, 0});
         }
     }
-    void build_tasks2d_() {
+    void draw_tasks2d() {
         // interior: R cells clear of the padding and off the outer (Dirichlet) ring
         const int xa = pl[0] > 0 ? pl[0] + R : 1;
         const int xb = pr[0] > 0 ? nx - pr[0] - R : nx - 1;
@@ -654,6 +658,13 @@ struct PlanT final : public pysit_plan {
         if (kind == 0 && tz > 0) w = std::min(w, tz);
         split3d(za, zb, w, zs);
         const int nxc = (xb - xa + tx - 1) / tx, wx = (xb - xa + nxc - 1) / nxc;
+        if (counting) {
+            for (auto& z : zs) {
+                const int rows = wave3d_task_rows((int)sizeof(T), threads3d, z.second - z.first);
+                counted += (size_t)((xb - xa + wx - 1) / wx) * ((yb - ya + rows - 1) / rows);
+            }
+            return;
+        }
         for (int x = xa; x < xb; x += wx)
             for (auto& z : zs) {
                 const int nzv = (z.second - z.first + V - 1) / V;
@@ -684,24 +695,22 @@ struct PlanT final : public pysit_plan {
     void build_tasks3d() {
         const int keep = tx;
         for (;; tx = std::max(1, tx / 2)) {  // shorter tiles until every tile's injection fits
-            build_tasks3d_();
+            tasks3d.clear();
+            tiles3d.clear();
+            draw_tasks3d();
             if (size_tiles3d() || tx == 1) break;
         }
         tx = keep;
     }
-    void build_tasks3d_() {
-        tasks3d.clear();
-        tiles3d.clear();
+    void draw_tasks3d() {
         const int xa = pl[0] > 0 ? pl[0] + R : 1, xb = pr[0] > 0 ? nx - pr[0] - R : nx - 1;
         const int ya = pl[1] > 0 ? pl[1] + R : 1, yb = pr[1] > 0 ? ny - pr[1] - R : ny - 1;
         const int za = ((pl[2] > 0 ? pl[2] + R : 1) + 3) / 4 * 4;
         const int zb = (pr[2] > 0 ? nz - pr[2] - R : nz - 1) / 4 * 4;
-        ntask3d[0] = ntask3d[1] = 0;
         if (xa >= xb || ya >= yb || za >= zb) {
             add_tasks3d(0, nx, 0, ny, 0, nz, 1);
         } else {
             add_tasks3d(xa, xb, ya, yb, za, zb, 0);
-            ntask3d[0] = (int)tiles3d.size();
             // off the padding: y in [y0, y1); z in [z0, z1) (multiples of 4, or the grid's end)
             const int y0 = pl[1], y1 = ny - pr[1];
             const int z0 = (pl[2] + 3) / 4 * 4, z1 = pr[2] > 0 ? (nz - pr[2]) / 4 * 4 : nz;
@@ -721,23 +730,27 @@ struct PlanT final : public pysit_plan {
                 add_tasks3d(xa, xb, ya, yb, side ? zb : 0, side ? nz : za, 4);
             }
         }
-        ntask3d[1] = (int)tiles3d.size() - ntask3d[0];
     }
 
-    // ints of the task table for a task length tx_try and z extent tz_try (the current table is kept)
+    // tiles of the task table for a task length tx_try and z extent tz_try, counted only: the table with
+    // its injection boxes takes milliseconds to build (1000 shots of 1232 x 464: 166 ms a plan when the
+    // largest table was found by building each)
     static constexpr int kMinTileX = 8;
     static constexpr int kMinTileZ = 16;
-    size_t task_ints(int tx_try, int tz_try) {
-        if (dim == 1) return 0;
+    bool counting = false;
+    size_t counted = 0;
+    size_t count_tasks(int tx_try, int tz_try) {
         const int keep = tx, keepz = tz;
         tx = tx_try;
         tz = tz_try;
-        size_t n;
-        if (dim == 2) { build_tasks2d(); n = tasks2d.size(); } else { build_tasks3d(); n = tasks3d.size(); }
+        counting = true;
+        counted = 0;
+        if (dim == 2) draw_tasks2d();
+        if (dim == 3) draw_tasks3d();
+        counting = false;
         tx = keep;
         tz = keepz;
-        if (dim == 2) build_tasks2d(); else build_tasks3d();
-        return n;
+        return counted;
     }
 
     long long internal_offset(long long cell) const {
@@ -874,9 +887,11 @@ struct PlanT final : public pysit_plan {
         // the largest table any tuning can ask for: the shortest x-chunk, and every z extent
         // (in 3D a narrower segment can give more tasks: its warps take several rows, but
         // not always enough to make up for the extra segments)
-        task_cap = std::max<size_t>(task_ints(kMinTileX, 0), std::max(tasks2d.size(), tasks3d.size()));
-        for (int z = kMinTileZ; z <= 32 * V16<T>::N; z += 4) task_cap = std::max(task_cap, task_ints(kMinTileX, z));
-        off.tasks = take(std::max<size_t>(dim == 2 ? task_cap / 5 * sizeof(Tile2d) : task_cap / 6 * sizeof(Tile3d), sizeof(Tile3d)));
+        // (3D: injections that do not fit shorten the tiles, to one plane at most)
+        const int shortest = dim == 3 ? 1 : kMinTileX;
+        task_cap = std::max(count_tasks(shortest, 0), dim == 3 ? tiles3d.size() : tiles2d.size());
+        for (int z = kMinTileZ; z <= 32 * V16<T>::N; z += 4) task_cap = std::max(task_cap, count_tasks(shortest, z));
+        off.tasks = take((task_cap + 1) * (dim == 3 ? sizeof(Tile3d) : sizeof(Tile2d)));
         off.partial = take(kRedBlocks * sizeof(double));
         off.rnorm = take(sizeof(double));
         ws_need = tot;
@@ -1562,8 +1577,10 @@ struct PlanT final : public pysit_plan {
     int use_tile(int t, int z, cudaStream_t s) {
         tx = t;
         tz = z > 0 ? z / 4 * 4 : 0;
-        std::vector<int>& tab = dim == 3 ? (build_tasks3d(), tasks3d) : (build_tasks2d(), tasks2d);
-        PGB_REQUIRE(tab.size() <= task_cap, "task table of %zu ints exceeds its buffer (%zu)", tab.size(), task_cap);
+        if (dim == 3) build_tasks3d();
+        else build_tasks2d();
+        const size_t n = dim == 3 ? tiles3d.size() : tiles2d.size();
+        PGB_REQUIRE(n <= task_cap, "task table of %zu tiles exceeds its buffer (%zu)", n, task_cap);
         int rc = dim == 3 ? upload(off.tasks, tiles3d, s) : upload(off.tasks, tiles2d, s);
         if (rc) return rc;
         PGB_CHECK_CUDA(cudaStreamSynchronize(s));
