@@ -701,6 +701,8 @@ struct PlanT final : public pysit_plan {
             if (size_tiles3d() || tx == 1) break;
         }
         tx = keep;
+        ntask3d[0] = (int)std::count_if(tiles3d.begin(), tiles3d.end(), [](const Tile3d& t) { return t.kind == 0; });
+        ntask3d[1] = (int)tiles3d.size() - ntask3d[0];
     }
     void draw_tasks3d() {
         const int xa = pl[0] > 0 ? pl[0] + R : 1, xb = pr[0] > 0 ? nx - pr[0] - R : nx - 1;
