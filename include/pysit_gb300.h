@@ -273,16 +273,17 @@ int pysit_plan_step_loop(pysit_plan* plan, int mode, int nsteps, void* stream);
 
 /* Autotuner, no counterpart in the reference (its kernels have no tiles): times
  * `nsteps` forward and `nsteps` adjoint steps (as pysit_plan_step_loop does) for
- * each of the `ncand` task lengths along x in `candidates` (8..4096 rows), twice (the
- * second pass in reverse order), keeps the fastest, writes it to *chosen and the
+ * each of the `ncand` task lengths along x in `candidates` (0 = the plan's default, else 8..4096
+ * rows in 2D, 1..4096 planes in 3D), twice (the second pass in reverse order; lengths that give
+ * the same table once for all), keeps the fastest, writes it to *chosen and the
  * better of each candidate's two times in milliseconds to ms[ncand] (may be NULL).  Needs a bound workspace and a model; 2D and 3D plans.
  * It drops the plan's captured graphs (they hold the old task tables); the
  * wavefield buffers are left in an arbitrary state, as after step_loop. */
 int pysit_plan_autotune(pysit_plan* plan, const int* candidates, int ncand, int nsteps, int* chosen,
                         double* ms, void* stream);
 /* The autotuner over both tile dimensions, no counterpart in the reference: as
- * pysit_plan_autotune for every pair of a task length along x in cand_x[ncx] (8..4096) and a
- * z extent of the interior tasks in cand_z[ncz] (0 = the full width, else >= 16 cells);
+ * pysit_plan_autotune for every pair of a task length along x in cand_x[ncx] (0 = the plan's default,
+ * else 8..4096 in 2D, 1..4096 in 3D) and a z extent of the interior tasks in cand_z[ncz] (0 = the full width, else >= 16 cells);
  * writes the fastest pair to *chosen_x / *chosen_z and the better of each pair's two times
  * to ms[ix * ncz + iz] (may be NULL). */
 int pysit_plan_autotune_tiles(pysit_plan* plan, const int* cand_x, int ncx, const int* cand_z, int ncz,

@@ -320,7 +320,8 @@ struct PlanT final : public pysit_plan {
     // ---- layout --------------------------------------------------------------
     int hx, hy, rows_y, ldz;
     long long fstride;  // elements per field per shot (256-byte multiple)
-    int tx;  // rows along x of a tile
+    int tx;      // rows along x of a tile at most
+    int def_tx;  // the rule's choice of it (tile_x 0)
     int nseg;
     std::vector<int> tasks2d;    // [ntasks][5] tiles of the 2D step: interior first, then shell
     int ntask2d[2] = {0, 0};     // tasks of each kind
@@ -489,7 +490,7 @@ struct PlanT final : public pysit_plan {
     }
 
     void choose_tiling() {
-        tx = 32;  // 1D has no tiles
+        tx = def_tx = 32;  // 1D has no tiles
         if (dim == 2) {
             if (tile_req) tx = tile_req;
             strip2d = choose_strip2d();
@@ -641,6 +642,7 @@ struct PlanT final : public pysit_plan {
         if (planes3d > 1)
             for (tx = 4; tx < 16 && blocks / (2 * tx) >= 4 * 304; tx *= 2) {}
         threads3d = planes3d > 1 ? kT3 : 64;
+        def_tx = tx;
         if (tile_req) tx = tile_req;
     }
 
@@ -737,8 +739,8 @@ struct PlanT final : public pysit_plan {
     // tiles of the task table for a task length tx_try and z extent tz_try, counted only: the table with
     // its injection boxes takes milliseconds to build (1000 shots of 1232 x 464: 166 ms a plan when the
     // largest table was found by building each)
-    static constexpr int kMinTileX = 8;
     static constexpr int kMinTileZ = 16;
+    int min_tile_x() const { return dim == 3 ? 1 : 8; }  // shortest that the tuner takes
     bool counting = false;
     size_t counted = 0;
     size_t count_tasks(int tx_try, int tz_try) {
@@ -889,10 +891,8 @@ struct PlanT final : public pysit_plan {
         // the largest table any tuning can ask for: the shortest x-chunk, and every z extent
         // (in 3D a narrower segment can give more tasks: its warps take several rows, but
         // not always enough to make up for the extra segments)
-        // (3D: injections that do not fit shorten the tiles, to one plane at most)
-        const int shortest = dim == 3 ? 1 : kMinTileX;
-        task_cap = std::max(count_tasks(shortest, 0), dim == 3 ? tiles3d.size() : tiles2d.size());
-        for (int z = kMinTileZ; z <= 32 * V16<T>::N; z += 4) task_cap = std::max(task_cap, count_tasks(shortest, z));
+        task_cap = std::max(count_tasks(min_tile_x(), 0), dim == 3 ? tiles3d.size() : tiles2d.size());
+        for (int z = kMinTileZ; z <= 32 * V16<T>::N; z += 4) task_cap = std::max(task_cap, count_tasks(min_tile_x(), z));
         off.tasks = take((task_cap + 1) * (dim == 3 ? sizeof(Tile3d) : sizeof(Tile2d)));
         off.partial = take(kRedBlocks * sizeof(double));
         off.rnorm = take(sizeof(double));
@@ -1502,7 +1502,8 @@ struct PlanT final : public pysit_plan {
     }
 
     // Every (x length, z extent) pair is timed twice, the second pass in reverse order; each
-    // keeps its faster time and the fastest pair stays.  ms_out[ix * ncz + iz].
+    // keeps its faster time and the fastest pair stays.  Pairs that give the same table (2D lengths
+    // beyond a block's rows) are timed once, and the first of them stands for all.  ms_out[ix * ncz + iz].
     int autotune2(const int* cx, int ncx, const int* cz, int ncz, int n, int* chosen_x, int* chosen_z,
                   double* ms_out, cudaStream_t s) override {
         PGB_REQUIRE(ws, "no workspace bound");
@@ -1511,8 +1512,8 @@ struct PlanT final : public pysit_plan {
         PGB_REQUIRE(cx && ncx >= 1 && cz && ncz >= 1 && chosen_x && chosen_z, "need candidates and outputs");
         PGB_REQUIRE(n >= 1, "nsteps must be >= 1");
         for (int c = 0; c < ncx; ++c)
-            PGB_REQUIRE(cx[c] >= kMinTileX && cx[c] <= 4096, "candidate task length %d outside [%d, 4096]", cx[c],
-                        kMinTileX);
+            PGB_REQUIRE(cx[c] == 0 || (cx[c] >= min_tile_x() && cx[c] <= 4096),
+                        "candidate task length %d outside [%d, 4096] (0: the default)", cx[c], min_tile_x());
         for (int c = 0; c < ncz; ++c)
             PGB_REQUIRE(cz[c] == 0 || cz[c] >= kMinTileZ, "candidate z extent %d below %d (0: full width)", cz[c],
                         kMinTileZ);
@@ -1524,10 +1525,21 @@ struct PlanT final : public pysit_plan {
         float best_ms = 1e30f;
         int rc = PYSIT_OK;
         std::vector<float> t(nc, 1e30f);
+        std::vector<int> first(nc);           // the first pair with the pair's table
+        std::vector<std::vector<int>> table(nc);
         for (int pass = 0; pass < 2 && rc == PYSIT_OK; ++pass)
             for (int i = 0; i < nc && rc == PYSIT_OK; ++i) {
                 const int c = pass == 0 ? i : nc - 1 - i;
+                if (pass == 1 && first[c] != c) continue;
                 if ((rc = use_tile(cx[c / ncz], cz[c % ncz], s))) break;
+                if (pass == 0) {
+                    table[c] = dim == 3 ? tasks3d : tasks2d;
+                    first[c] = (int)(std::find(table.begin(), table.begin() + c, table[c]) - table.begin());
+                    if (first[c] != c) {
+                        table[c].clear();
+                        continue;
+                    }
+                }
                 // the sweeps a gradient runs: forward (in recompute mode when dWaveOp is kept) and adjoint
                 const int fmode = store_all ? kRecomp : kFwd;
                 if ((rc = step_loop(fmode, 2, s))) break;  // warm-up
@@ -1540,6 +1552,7 @@ struct PlanT final : public pysit_plan {
                 t[c] = std::min(t[c], ms);
             }
         for (int c = 0; c < nc && rc == PYSIT_OK; ++c) {
+            t[c] = t[first[c]];
             if (ms_out) ms_out[c] = t[c];
             if (t[c] < best_ms) { best_ms = t[c]; best = c; }
         }
@@ -1574,10 +1587,10 @@ struct PlanT final : public pysit_plan {
         return PYSIT_OK;
     }
 
-    // rebuild and upload the task table for task length t and z extent z; captured graphs
+    // rebuild and upload the task table for task length t (0: the default) and z extent z; captured graphs
     // hold the old table's counts, so they are dropped
     int use_tile(int t, int z, cudaStream_t s) {
-        tx = t;
+        tx = t > 0 ? t : def_tx;
         tz = z > 0 ? z / 4 * 4 : 0;
         if (dim == 3) build_tasks3d();
         else build_tasks2d();

@@ -34,7 +34,9 @@ _DESC_AXIS = {1: [2], 2: [0, 2], 3: [0, 1, 2]}  # mesh axis -> (x, y, z) slot of
 # use and written back after every new tuning, so later processes on the machine start from it.
 _TUNED = {}
 _TUNE_FILES_READ = set()
-TILE_CANDIDATES = {2: (8, 16, 32, 64), 3: (8, 16, 32, 64)}
+# task lengths along x tried; 0 stands for the plan's default, which depends on the launch's cells
+# (1 to 16 planes in 3D) and so is always among them
+TILE_CANDIDATES = {2: (0, 8, 16, 32, 64), 3: (0, 1, 4, 8, 16, 32, 64)}
 # z extents of the interior tasks tried, as fractions of the kernels' full width (32 lanes x
 # the 16-byte lane vector: 128 cells in FP32, 64 in FP64); 0 stands for the full width
 TILE_Z_FRACTIONS = (1.0, 0.75, 0.5)
@@ -455,8 +457,8 @@ class WavePlan:
         """Time every pair of a task length along x in `candidates` and a z extent of the
         interior tasks in `z_candidates` (0: the full width; forward + adjoint steps on this
         plan's buffers), keep the fastest for this plan and for later plans of the same
-        configuration.  Returns {"chosen": rows, "chosen_z": cells, "ms": {(x, z): milliseconds}}.
-        1D plans have no tiles."""
+        configuration.  Returns {"chosen": rows (0: the plan's default), "chosen_z": cells,
+        "ms": {(x, z): milliseconds}}.  1D plans have no tiles."""
         if self.dim == 1:
             return {"chosen": 0, "chosen_z": 0, "ms": {}}
         torch = _native.require_cuda()

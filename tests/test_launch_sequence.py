@@ -65,3 +65,42 @@ def test_bind_returns_with_the_workspace_complete(fake, dim, n):
     work = [i for i, l in enumerate(out) if l.split()[0] in ("launch", "memcpy", "memset")]
     assert any("one_sigma" in out[i] for i in work)
     assert "sync 7" in out[work[-1] + 1:]
+
+
+TUNE = """
+d = _desc(keep, {dim}, {n}, ((4, 4),) * 3, 4, _native.PYSIT_F64)
+h = plan(d); model(h, d)
+tile = C.c_int(); _native.check(lib.pysit_plan_get_tiles(h, C.byref(tile), None)); before = tile.value
+cx, cz = (C.c_int * {nx})(*{cx}), (C.c_int * 1)(0)
+x, z, ms = C.c_int(), C.c_int(), (C.c_double * {nx})()
+fake.fake_clear()
+_native.check(lib.pysit_plan_autotune_tiles(h, cx, {nx}, cz, 1, 3, C.byref(x), C.byref(z), ms, C.c_void_p(7)))
+_native.check(lib.pysit_plan_get_tiles(h, C.byref(tile), None))
+print(before, x.value, tile.value, sum(l.startswith("record") for l in log()) // 2, *ms)
+"""
+
+
+@pytest.mark.parametrize("times,chosen", [("1,2,2,1", 0), ("2,1,1,2", 8)])
+def test_the_tuner_may_keep_the_default_length(fake, times, chosen):
+    """A small 3D plan's default of one plane is a candidate (0), kept when it is the fastest."""
+    out = _run(fake, TUNE.format(dim=3, n=(20, 18, 24), nx=2, cx=(0, 8)), FAKE_MS=times)
+    before, x, tile, timed, *ms = out[-1].split()
+    assert int(before) == 1 and int(x) == chosen and int(tile) == (chosen or 1)
+    assert int(timed) == 4 and [float(v) for v in ms] == [float(v) for v in times.split(",")[:2]]
+
+
+def test_the_3d_tuner_takes_lengths_down_to_one_plane(fake):
+    out = _run(fake, TUNE.format(dim=3, n=(20, 18, 24), nx=4, cx=(64, 4, 2, 1)), FAKE_MS="4,3,2,1,1,2,3,4")
+    assert out[-1].split()[:4] == ["1", "1", "1", "8"]
+
+
+def test_lengths_that_give_the_same_2d_table_are_timed_once(fake):
+    # blocks of three rows: every length gives the same tiles
+    out = _run(fake, TUNE.format(dim=2, n=(300, 1, 36), nx=4, cx=(8, 64, 200, 0)), FAKE_MS="2,1")
+    before, x, tile, timed, *ms = out[-1].split()
+    assert (int(before), int(x), int(timed)) == (32, 8, 2) and [float(v) for v in ms] == [1, 1, 1, 1]
+
+
+def test_the_tuner_tries_the_default():
+    from pysit_gb300 import engine
+    assert all(c[0] == 0 for c in engine.TILE_CANDIDATES.values()) and 1 in engine.TILE_CANDIDATES[3]
