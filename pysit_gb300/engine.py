@@ -28,12 +28,15 @@ __all__ = ["WavePlan", "PlanGroup", "padded_cells", "default_checkpoint_every"]
 _DESC_AXIS = {1: [2], 2: [0, 2], 3: [0, 1, 2]}  # mesh axis -> (x, y, z) slot of the descriptor
 
 # tunings chosen by WavePlan.autotune (task length along x, 2D shell block shares per step
-# mode, z extent of the interior tasks), per (dim, order, padded grid, dtype, psi form, shots per launch, schedule, forward
+# mode, z extent of the interior tasks), per (kernels, dim, order, padded grid, dtype, psi form, shots per launch, schedule, forward
 # only, lanes); later plans of the same configuration start from them.  With the environment
 # variable PYSIT_CUDA_TUNE_CACHE naming a JSON file, the table is read from that file on first
 # use and written back after every new tuning, so later processes on the machine start from it.
 _TUNED = {}
 _TUNE_FILES_READ = set()
+# which step kernels a tuning was timed on: changed with their tiles, so that a file written for other
+# kernels (whose best 3D length, 64 planes, is a tenth and more slower on these) is not applied
+_TILES = "tiles-2"
 # task lengths along x tried; 0 stands for the plan's default, which depends on the launch's cells
 # (1 to 16 planes in 3D) and so is always among them
 TILE_CANDIDATES = {2: (0, 8, 16, 32, 64), 3: (0, 1, 4, 8, 16, 32, 64)}
@@ -100,6 +103,11 @@ def _tuning_put(key, value):
     path = _tune_cache_file()
     if path:
         _write_tunings(path, {**_read_tunings(path), **_TUNED})
+
+
+def _tuning_key(dim, order, shape, dtype, psi_consistent, shots_per_launch, schedule, forward_only, lanes):
+    return (_TILES, dim, order, tuple(shape), str(dtype), psi_consistent, shots_per_launch, schedule, forward_only,
+            lanes)
 
 
 def padded_cells(mesh, cells):
@@ -204,8 +212,6 @@ class WavePlan:
         d.psi_consistent = 1 if getattr(solver, "pml_psi", "reference") == "consistent" else 0
         d.wait_polls = int(wait_polls)
         d.wait_fault = 1 if wait_fault else 0
-        self._tune_key = (self.dim, solver.spatial_accuracy_order, tuple(full), str(solver.dtype),
-                          d.psi_consistent)
         self.record_steps = None
         if record_steps is not None:
             rs = np.ascontiguousarray(np.asarray(record_steps, dtype=np.int32).reshape(-1))
@@ -261,7 +267,8 @@ class WavePlan:
         d.shots_per_launch = self.shots_per_launch
         self.gradient_schedule = gradient_schedule
         # the tuning key knows the launch size and schedule only now
-        self._tune_key = self._tune_key + (self.shots_per_launch, gradient_schedule, self.forward_only, self.lanes)
+        self._tune_key = _tuning_key(self.dim, solver.spatial_accuracy_order, full, solver.dtype, d.psi_consistent,
+                                     self.shots_per_launch, gradient_schedule, self.forward_only, self.lanes)
         tuned = _tuning_get(self._tune_key)
         d.tile_x = tuned[0] if tuned else 0
         for k in range(3):
