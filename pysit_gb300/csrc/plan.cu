@@ -363,6 +363,10 @@ struct PlanT final : public pysit_plan {
     // leaves the GPU idle recomputes a segment beside the adjoint steps of the segment after it, on
     // a second stream and into a second replay buffer.  (1D and small 3D launches do both; small 2D
     // launches keep a recompute step for every step.)
+    // A second replay buffer takes a GiB at most: a caller that asks for longer segments on a small
+    // launch chose checkpoints to save memory (two shots of 1232 x 464 with S = 2000 would hold 19 GB of
+    // replay instead of 9.6), and plans sized to the free memory leave 2 GiB of it.
+    static constexpr size_t kMaxSecondReplay = (size_t)1 << 30;
     bool overlap = false, keep_last = false;
     cudaStream_t aux = nullptr;  // the recompute steps' stream when they overlap
     cudaEvent_t ev_fork = nullptr, ev_ready[2] = {nullptr, nullptr}, ev_free[2] = {nullptr, nullptr};
@@ -468,7 +472,7 @@ struct PlanT final : public pysit_plan {
         sweeps1d = dim == 1 && wave1d_sweeps<T>(nz, std::max(nsrc, nrec));
         const bool fills = dim == 2 ? (long long)nx * nz * G * (int)sizeof(T) >= 64LL * kT2 * 4 * 152 : dim == 3 && planes3d == 4;
         const bool ckpt = !store_all && !fwd_only;
-        overlap = ckpt && !fills && nseg > 1;
+        overlap = ckpt && !fills && nseg > 1 && field_bytes * (size_t)S <= kMaxSecondReplay;
         keep_last = ckpt && (fills || dim != 2);
         // acquisition
         int rc = build_injection(d.src_tap_ptr, d.src_tap_cell, d.src_tap_point, d.src_tap_w, nsrc,
