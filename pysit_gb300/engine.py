@@ -335,17 +335,14 @@ class WavePlan:
 
         def fit(store):
             """Largest balanced launch of this schedule within the budget (0: none fits)."""
-            b1 = self._workspace_for(lib, d, 1, store)
-            per = self._workspace_for(lib, d, 2, store) - b1
-            gmax = self.nshots if per <= 0 else int((budget - (b1 - per)) // per)
-            gmax = min(gmax, self.nshots)
-            if gmax < 1:
-                return 0
-            glane = max(1, min(gmax // lanes, per_lane))
-            g = -(-per_lane // -(-per_lane // glane))
-            while g > 1 and self._workspace_for(lib, d, g, store, lanes) > budget:
-                g -= 1
-            return g
+            # measured launch by launch: a workspace is no multiple of a shot's (small launches hold
+            # two replay buffers, larger ones one)
+            g = per_lane + 1
+            while g > 1:
+                g = -(-per_lane // -(-per_lane // (g - 1)))
+                if self._workspace_for(lib, d, g, store, lanes) <= budget:
+                    return g
+            return 0
 
         g = fit(True)
         if g >= min(8, self.nshots):
