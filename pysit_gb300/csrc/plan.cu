@@ -358,6 +358,7 @@ struct PlanT final : public pysit_plan {
     } off{};
     size_t field_bytes = 0;      // one field for G shots
     bool sweeps1d = false;       // 1D: runs of steps as one launch
+    int sweep_nc = 0;            // its blocks per shot at most
     // Checkpointed gradients.  A launch that fills the GPU runs the last segment of the forward sweep
     // in recompute mode, straight into the replay buffer (one segment less to recompute).  One that
     // leaves the GPU idle recomputes a segment beside the adjoint steps of the segment after it, on
@@ -469,7 +470,6 @@ struct PlanT final : public pysit_plan {
         nslots = store_all ? (nsteps + p_img - 1) / p_img : S;
         ckpt_fields = dim == 1 ? 3 : dim == 2 ? 4 : 6;
         choose_tiling();
-        sweeps1d = dim == 1 && wave1d_sweeps<T>(nz, std::max(nsrc, nrec));
         const bool fills = dim == 2 ? (long long)nx * nz * G * (int)sizeof(T) >= 64LL * kT2 * 4 * 152 : dim == 3 && planes3d == 4;
         const bool ckpt = !store_all && !fwd_only;
         overlap = ckpt && !fills && nseg > 1 && field_bytes * (size_t)S <= kMaxSecondReplay;
@@ -976,6 +976,15 @@ struct PlanT final : public pysit_plan {
             for (auto e : {&ev_fork, &ev_ready[0], &ev_ready[1], &ev_free[0], &ev_free[1]})
                 if (!*e) PGB_CHECK_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
         }
+        if (dim == 1 && wave1d_sweeps<T>(nz, nsrc, nrec, G)) {
+            switch (R) {
+                case 1: sweep_nc = wave1d_prepare<T, 1>(nz, nsrc, nrec); break;
+                case 2: sweep_nc = wave1d_prepare<T, 2>(nz, nsrc, nrec); break;
+                case 3: sweep_nc = wave1d_prepare<T, 3>(nz, nsrc, nrec); break;
+                default: sweep_nc = wave1d_prepare<T, 4>(nz, nsrc, nrec); break;
+            }
+            sweeps1d = sweep_nc > 0;  // a device that places no such cluster steps launch by launch
+        }
         if (dim == 3) switch (R) {
             case 1: wave3d_tile_prepare<T, 1>(); break;
             case 2: wave3d_tile_prepare<T, 2>(); break;
@@ -1189,6 +1198,7 @@ struct PlanT final : public pysit_plan {
         q.out_prev = own[0]; q.out_cur = own[1]; q.out_phz = own[2];
         q.k0 = k0; q.n = n; q.dir = dir;
         q.npts_max = std::max(nsrc, nrec);
+        q.most_nc = sweep_nc;
         q.field_stride = (long long)fstride * G;
         q.S = S;
         ++launches;

@@ -277,6 +277,7 @@ struct Sweep1d {
     T *out_prev, *out_cur, *out_phz;     // and after the last
     int k0, n, dir;                      // first step, number of steps, +1 or -1
     int npts, npts_max;                  // injection points of this run; of any run of the plan
+    int most_nc;                         // blocks per shot at most (wave1d_prepare)
     T* traces;                           // NULL, or the traces of step 0 of shot 0 (rows of p.rec.nrec)
     T* dw;                               // NULL, or dWaveOp: step k with k % dw_period == 0 in field (k - dw_k0) / dw_div
     int dw_period, dw_k0, dw_div;
@@ -284,10 +285,15 @@ struct Sweep1d {
     int S;
     long long field_stride;              // elements between fields of a launch's shots
     int cells, threads;                  // cells per block and threads that step them (set by the launch)
+    unsigned inv;                        // ceil(2^32 / cells): the block of a cell
 };
-// whether a grid of nz cells with at most npts injection points runs as sweeps
+// whether launches of nshot shots on a grid of nz cells run as sweeps
 template <typename T>
-bool wave1d_sweeps(int nz, int npts);
+bool wave1d_sweeps(int nz, int nsrc, int nrec, int nshot);
+// readies the kernels on the device; the largest cluster limit (16 or 8 blocks) whose clusters it places,
+// 0: none
+template <typename T, int R>
+int wave1d_prepare(int nz, int nsrc, int nrec);
 template <typename T, int R, int MODE>
 void launch_wave1d_sweep(const WaveParams<T>& p, Sweep1d<T> q, cudaStream_t s);
 template <typename T, int R, int MODE>

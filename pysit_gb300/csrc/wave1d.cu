@@ -8,7 +8,8 @@
 // Checkpoints, traces, dWaveOp and the image go to and come from global memory as the steps pass.
 // What bounds a step: in FP64 the few FP64 units of the cluster's SMs, then the barrier.  Measured
 // against one launch per step of one thread per cell (800 steps of 799 cells, order 4, FP64, whole
-// gradient call): 6.4 -> 4.0 ms.  Grids too long for a cluster step as before, one launch each.
+// gradient call): 6.4 -> 4.0 ms.  Grids too long for a cluster and launches that fill the GPU
+// (wave1d_sweeps) step as before, one launch each.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -175,24 +176,47 @@ __global__ void __launch_bounds__(kThreads1) wave1d_sweep_kernel(const WaveParam
             }
         }
         if (MODE != kAdj && rw >= 0 && q.traces) {
-            // traces of u_k, a warp per receiver, the blocks in turn: the lanes fetch the taps (from the
-            // block that holds their cell), lane by lane they are summed in order
-            for (int r = rank + nc * rw; r < p.rec.nrec; r += nc * nrw) {
-                const long long id = (long long)shot * p.rec.nrec + r;
-                const int lane = tid & 31, e1r = __ldg(p.rec.rowptr + id + 1);
-                T acc = T(0);
-                for (int e = __ldg(p.rec.rowptr + id); e < e1r; e += 32) {
-                    const int m = min(32, e1r - e);
-                    T wt = T(0), v = T(0);
-                    if (lane < m) {
-                        const int cell = (int)(__ldg(p.rec.off + e + lane) - kOZ), b = cell / q.cells;
-                        wt = __ldg(p.rec.w + e + lane);
-                        v = cl.map_shared_rank(u[0], b)[(uk - u[0]) + cell - b * q.cells];
+            // traces of u_k, each in the order of its taps, read from the block that holds their cell
+            auto sample = [&](int e, T& wt, T& v) {
+                const int cell = (int)(__ldg(p.rec.off + e) - kOZ), b = __umulhi(cell, q.inv);
+                wt = __ldg(p.rec.w + e);
+                const T* ub = b == rank ? u[0] : cl.map_shared_rank(u[0], b);
+                v = ub[(uk - u[0]) + cell - b * q.cells];
+            };
+            T* out = q.traces + (long long)shot * p.rec.tr_sstride + (long long)k * p.rec.nrec;
+            const int* row = p.rec.rowptr + (long long)shot * p.rec.nrec;
+            if (p.rec.nrec <= 4 * nc) {  // a warp per receiver: the lanes fetch its taps
+                const int r = rank + nc * rw, lane = tid & 31;
+                if (r < p.rec.nrec) {
+                    const int e1r = __ldg(row + r + 1);
+                    T acc = T(0);
+                    for (int e = __ldg(row + r); e < e1r; e += 32) {
+                        const int m = min(32, e1r - e);
+                        T wt = T(0), v = T(0);
+                        if (lane < m) sample(e + lane, wt, v);
+                        for (int t = 0; t < m; ++t)
+                            acc += __shfl_sync(0xffffffffu, wt, t) * __shfl_sync(0xffffffffu, v, t);
                     }
-                    for (int t = 0; t < m; ++t)
-                        acc += __shfl_sync(0xffffffffu, wt, t) * __shfl_sync(0xffffffffu, v, t);
+                    if (lane == 0) out[r] = acc;
                 }
-                if (lane == 0) q.traces[(long long)shot * p.rec.tr_sstride + (long long)k * p.rec.nrec + r] = acc;
+            } else {  // a thread per receiver, neighbouring receivers in one block
+                const int per = (p.rec.nrec + nc - 1) / nc, rend = min(p.rec.nrec, (rank + 1) * per);
+                for (int r = rank * per + tid - nt; r < rend; r += 32 * nrw) {
+                    const int e1r = __ldg(row + r + 1);
+                    T acc = T(0);
+                    for (int e = __ldg(row + r); e < e1r; e += 8) {  // eight taps in flight
+                        T wt[8], v[8];
+#pragma unroll
+                        for (int t = 0; t < 8; ++t) {
+                            wt[t] = v[t] = T(0);
+                            if (e + t < e1r) sample(e + t, wt[t], v[t]);
+                        }
+#pragma unroll
+                        for (int t = 0; t < 8; ++t)
+                            if (e + t < e1r) acc += wt[t] * v[t];
+                    }
+                    out[r] = acc;
+                }
             }
         }
         const bool img = q.dw && k % q.dw_period == 0;
@@ -255,50 +279,102 @@ __global__ void __launch_bounds__(kThreads1) wave1d_sweep_kernel(const WaveParam
     }
 }
 
-// blocks per shot and cells per block; 0 blocks: the grid or its point sets are too large for a cluster
+struct SweepShape {
+    int nc, cells, threads;  // blocks per shot (0: none fits), cells per block, threads that step them
+};
+// the shape for a grid of nz cells, at most npts points and clusters of at most `most_nc` blocks
 template <typename T>
-int sweep1d_shape(int nz, int npts, int* cells) {
+SweepShape sweep1d_shape(int nz, int npts, int most_nc) {
     // a block's cells: in FP64 as few as give a few warps (the FP64 units bound the step: 2.4 us a step at
     // 100 cells a block, 3.5 at 250, where a launch per step takes 3.0), with sixteen blocks where eight
-    // would hold more than 128 each; in FP32 a block's threads (1.5 us a step from 150 to 2000 cells)
+    // would hold more than 128 each; in FP32 a block's threads (1.5 us a step from 150 to 2000 cells);
+    // more blocks for more receivers than a block's recording threads take at once
     const int want = sizeof(T) == 8 ? 64 : 512, most = sizeof(T) == 8 ? 160 : 2048;
-    const int lim = sizeof(T) == 8 && nz > 8 * 128 ? 16 : 8;
-    int nc = std::min(lim, ceil_div(nz, want));
-    for (;; --nc) {
-        *cells = ceil_div(nz, nc);
-        if (nc == 1 || nz - (nc - 1) * *cells >= kH1) break;  // the last block feeds its neighbour's halo
+    const int lim = std::min(most_nc, sizeof(T) == 8 && nz > 8 * 128 ? 16 : 8);
+    SweepShape h{std::min({lim, std::max(ceil_div(nz, want), ceil_div(npts, 128)), ceil_div(nz, kH1)}), 0, 0};
+    if (h.nc < 1) return SweepShape{};
+    for (;; --h.nc) {
+        h.cells = ceil_div(nz, h.nc);
+        if (h.nc == 1 || nz - (h.nc - 1) * h.cells >= kH1) break;  // the last block feeds its neighbour's halo
     }
-    if (*cells > most || sweep1d_smem<T>(*cells, npts) > 200 * 1024) return 0;
-    return nc;
+    h.threads = std::min(kThreads1 - 128, (h.cells + 31) / 32 * 32);
+    if (h.cells > most || sweep1d_smem<T>(h.cells, npts) > 200 * 1024) return SweepShape{};
+    return h;
+}
+// recording threads of a block: a warp per receiver for a few, else a thread per receiver
+inline int sweep1d_recorders(const SweepShape& h, int nrec) {
+    if (nrec <= 4 * h.nc) return 32 * ceil_div(nrec, h.nc);
+    return std::min(kThreads1 - h.threads, (ceil_div(nrec, h.nc) + 31) / 32 * 32);
+}
+
+// launch configuration of a run (`attr`: room for its cluster attribute)
+template <typename T>
+cudaLaunchConfig_t sweep1d_config(const SweepShape& h, int nshot, int npts, int recorders, cudaLaunchAttribute* attr) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(h.nc * nshot);
+    cfg.blockDim = dim3(h.threads + recorders);
+    cfg.dynamicSmemBytes = sweep1d_smem<T>(h.cells, npts);
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim = {(unsigned)h.nc, 1, 1};
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// whether the device places a cluster of the shape in one mode; sets the kernel's attributes
+template <typename T, int R, int MODE>
+bool sweep1d_placed(const SweepShape& h, int npts, int recorders) {
+    if (sweep1d_smem<T>(h.cells, npts) > 48 * 1024 &&
+        cudaFuncSetAttribute(wave1d_sweep_kernel<T, R, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024))
+        return false;
+    if (h.nc > 8 && cudaFuncSetAttribute(wave1d_sweep_kernel<T, R, MODE>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1))
+        return false;
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = sweep1d_config<T>(h, 1, npts, recorders, &attr);
+    int n = 0;
+    return cudaOccupancyMaxActiveClusters(&n, wave1d_sweep_kernel<T, R, MODE>, &cfg) == cudaSuccess && n > 0;
 }
 
 }  // namespace
 
+// Large launches step faster with a launch per step, whose blocks share the whole GPU: a run's blocks meet
+// every step, and each reads the amplitudes of all receivers.  Measured against a launch per step (us a
+// step of the whole gradient call): FP64 799 cells x 64 shots (65536 threads) 13.0 against 13.1, 96 shots
+// 18.0 against 16.9, 32 shots 8.2 against 10.9; FP32 1520 x 96 (110592 threads) 6.9 against 8.0, 2220 x 64
+// (122880) 8.3 against 7.8.  Receivers: FP64 799 x 32 shots x 400 (102400 of them times blocks) 9.3
+// against 12.0, 64 shots (204800) 19.1 against 15.1; FP32 799 x 96 x 400 (153600) 7.2 against 8.4, 128
+// shots (204800) 10.3 against 8.9.
 template <typename T>
-bool wave1d_sweeps(int nz, int npts) {
-    int cells;
-    return sweep1d_shape<T>(nz, npts, &cells) > 0;
+bool wave1d_sweeps(int nz, int nsrc, int nrec, int nshot) {
+    const SweepShape h = sweep1d_shape<T>(nz, std::max(nsrc, nrec), 16);
+    const long long blocks = (long long)h.nc * nshot;
+    return h.nc > 0 && blocks * h.threads <= (sizeof(T) == 8 ? 65536 : 152 * 768) &&
+           blocks * nrec <= (sizeof(T) == 8 ? 120000 : 180000);
+}
+
+template <typename T, int R>
+int wave1d_prepare(int nz, int nsrc, int nrec) {
+    for (int most_nc : {16, 8}) {
+        const SweepShape h = sweep1d_shape<T>(nz, std::max(nsrc, nrec), most_nc);
+        if (h.nc > 0 && sweep1d_placed<T, R, kFwd>(h, nsrc, sweep1d_recorders(h, nrec)) &&
+            sweep1d_placed<T, R, kRecomp>(h, nsrc, sweep1d_recorders(h, nrec)) && sweep1d_placed<T, R, kAdj>(h, nrec, 0))
+            return most_nc;
+    }
+    cudaGetLastError();  // an attribute or shape that the device refuses is no error of the plan
+    return 0;
 }
 
 template <typename T, int R, int MODE>
 void launch_wave1d_sweep(const WaveParams<T>& p, Sweep1d<T> q, cudaStream_t s) {
-    const int nc = sweep1d_shape<T>(p.nz, q.npts_max, &q.cells);
+    const SweepShape h = sweep1d_shape<T>(p.nz, q.npts_max, q.most_nc);
     if (!p.inj.on) q.npts = 0;
-    const size_t smem = sweep1d_smem<T>(q.cells, q.npts);
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(wave1d_sweep_kernel<T, R, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (nc > 8) cudaFuncSetAttribute(wave1d_sweep_kernel<T, R, MODE>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(nc * p.nshot);
-    q.threads = std::min(kThreads1 - 128, (q.cells + 31) / 32 * 32);
-    cfg.blockDim = dim3(q.threads + (MODE != kAdj && q.traces ? 32 * std::min(4, ceil_div(p.rec.nrec, nc)) : 0));
-    cfg.dynamicSmemBytes = smem;
+    q.cells = h.cells;
+    q.threads = h.threads;
+    q.inv = 0xffffffffu / (unsigned)q.cells + 1;
+    cudaLaunchAttribute attr;
+    cudaLaunchConfig_t cfg =
+        sweep1d_config<T>(h, p.nshot, q.npts, MODE != kAdj && q.traces ? sweep1d_recorders(h, p.rec.nrec) : 0, &attr);
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim = {(unsigned)nc, 1, 1};
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, wave1d_sweep_kernel<T, R, MODE>, p, q);
 }
 
@@ -311,9 +387,10 @@ void launch_wave1d(const WaveParams<T>& p, cudaStream_t s) {
     wave1d_kernel<T, R, MODE><<<grid, tb, 0, s>>>(p, ntile);
 }
 
-template bool wave1d_sweeps<float>(int, int);
-template bool wave1d_sweeps<double>(int, int);
+template bool wave1d_sweeps<float>(int, int, int, int);
+template bool wave1d_sweeps<double>(int, int, int, int);
 #define PGB_INST1(T, R)                                                                  \
+    template int wave1d_prepare<T, R>(int, int, int);                                                 \
     template void launch_wave1d_sweep<T, R, kFwd>(const WaveParams<T>&, Sweep1d<T>, cudaStream_t);    \
     template void launch_wave1d_sweep<T, R, kRecomp>(const WaveParams<T>&, Sweep1d<T>, cudaStream_t); \
     template void launch_wave1d_sweep<T, R, kAdj>(const WaveParams<T>&, Sweep1d<T>, cudaStream_t);    \

@@ -104,3 +104,37 @@ def test_lengths_that_give_the_same_2d_table_are_timed_once(fake):
 def test_the_tuner_tries_the_default():
     from pysit_gb300 import engine
     assert all(c[0] == 0 for c in engine.TILE_CANDIDATES.values()) and 1 in engine.TILE_CANDIDATES[3]
+
+
+@pytest.mark.parametrize("nz,dtype,largest,cluster", [(1500, "F64", 16, 16), (1500, "F64", 8, 0), (1200, "F64", 16, 16),
+                                                      (1200, "F64", 8, 8), (1200, "F64", 0, 0), (300, "F32", 16, 1),
+                                                      (300, "F32", 0, 0)])
+def test_1d_runs_use_a_cluster_that_the_device_places(fake, nz, dtype, largest, cluster):
+    """Where the device places no cluster of a run's size, a smaller one is taken, or a launch per step."""
+    out = _run(fake, f"d = _desc(keep, 1, (1, 1, {nz}), ((0, 0), (0, 0), (9, 9)), 4, _native.PYSIT_{dtype})\n"
+                     "h = plan(d); model(h, d); fake.fake_clear()\n"
+                     "tr = np.zeros(8)\n"
+                     "_native.check(lib.pysit_plan_forward(h, C.c_void_p(tr.ctypes.data), C.c_void_p(7)))\n"
+                     "print('\\n'.join(log()))", FAKE_MAX_CLUSTER=str(largest))
+    runs = [l for l in out if "wave1d_sweep_kernel" in l]
+    steps = [l for l in out if "wave1d_kernel" in l]
+    assert [int(l.split()[-1]) for l in runs] == ([cluster] if cluster else [])
+    assert len(steps) == (0 if cluster else 8)
+
+
+@pytest.mark.parametrize("nshots,dtype,runs", [(64, "F64", 1), (128, "F64", 0), (128, "F32", 1), (512, "F32", 0)])
+def test_1d_launches_that_fill_the_gpu_step_one_launch_at_a_time(fake, nshots, dtype, runs):
+    out = _run(fake, f"d = _desc(keep, 1, (1, 1, 799), ((0, 0), (0, 0), (10, 10)), 4, _native.PYSIT_{dtype})\n"
+                     f"n = {nshots}\nd.nshots = d.shots_per_launch = n\n"
+                     "ptr = np.arange(n + 1, dtype=np.int64); one = np.ones(n); pt = np.zeros(n, np.int32)\n"
+                     "cell = np.full(n, 400, np.int64); amp = np.ones((n, 8, 1))\n"
+                     "P = lambda a, t: a.ctypes.data_as(C.POINTER(t))\n"
+                     "d.src_tap_ptr = d.rec_tap_ptr = P(ptr, C.c_int64); d.src_tap_cell = d.rec_tap_cell = P(cell, C.c_int64)\n"
+                     "d.src_tap_point = d.rec_tap_point = P(pt, C.c_int32); d.src_amp = P(amp, C.c_double)\n"
+                     "d.src_tap_w = d.rec_tap_wsample = d.rec_tap_winject = P(one, C.c_double)\n"
+                     "h = plan(d); model(h, d); fake.fake_clear()\n"
+                     "tr = np.zeros(8 * n)\n"
+                     "_native.check(lib.pysit_plan_forward(h, C.c_void_p(tr.ctypes.data), C.c_void_p(7)))\n"
+                     "print('\\n'.join(log()))")
+    assert sum("wave1d_sweep_kernel" in l for l in out) == runs
+    assert sum("wave1d_kernel" in l for l in out) == (0 if runs else 8)
