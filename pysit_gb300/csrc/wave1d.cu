@@ -117,9 +117,11 @@ __global__ void __launch_bounds__(kThreads1) wave1d_sweep_kernel(const WaveParam
     const int a = rank * q.cells, n = min(q.cells, p.nz - a);  // the block's cells a .. a+n-1
     const int w = q.cells + 2 * kH1, tid = threadIdx.x, nt = q.threads;  // nt threads step cells, the warps after them record
     const int rw = (tid - nt) >> 5, nrw = (blockDim.x - nt) >> 5;
-    T* u[2] = {reinterpret_cast<T*>(smem_raw) + kH1, reinterpret_cast<T*>(smem_raw) + w + kH1};  // u[cur], u[cur ^ 1] = u_{k-1} -> u_{k+1}
-    T* ph[2] = {u[0] + 2 * w, u[0] + 3 * w};
-    T* c2 = u[0] + 4 * w - kH1;
+    // u and Phi_z, each twice, w apart: `cur` (0 or w) is the offset of u_k and Phi_k, w - cur that of
+    // u_{k-1} -> u_{k+1} and Phi_{k+1}
+    T* const us = reinterpret_cast<T*>(smem_raw) + kH1;
+    T* const ps = us + 2 * w;
+    T* c2 = us + 4 * w - kH1;
     T *sg = c2 + q.cells, *mg = sg + q.cells, *fc = mg + q.cells, *ic = fc + q.cells, *amp = ic + q.cells;
     int* e0 = reinterpret_cast<int*>(amp + kAmpSteps * q.npts);
     int* e1 = e0 + q.cells;
@@ -127,10 +129,10 @@ __global__ void __launch_bounds__(kThreads1) wave1d_sweep_kernel(const WaveParam
     const int* bx = p.inj.box + shot * 6;
     // the state with its halos (zero beyond the grid: the fields' own zero halos)
     for (int j = tid - kH1; j < n + kH1; j += blockDim.x) {
-        u[0][j] = q.in_cur[sh + a + j];
-        u[1][j] = j >= 0 && j < n ? q.in_prev[sh + a + j] : T(0);
-        ph[0][j] = q.in_phz[sh + a + j];
-        ph[1][j] = T(0);
+        us[j] = q.in_cur[sh + a + j];
+        us[w + j] = j >= 0 && j < n ? q.in_prev[sh + a + j] : T(0);
+        ps[j] = q.in_phz[sh + a + j];
+        ps[w + j] = T(0);
     }
     for (int j = tid; j < n; j += blockDim.x) {
         const int k = a + j;
@@ -146,8 +148,8 @@ __global__ void __launch_bounds__(kThreads1) wave1d_sweep_kernel(const WaveParam
     }
     // the neighbours' halos: cells j < R go to the left block's right halo, cells j >= n-R to the right's left
     const int nl = q.cells;  // cells of the left neighbour (only the last block may have fewer)
-    T* left = rank > 0 ? cl.map_shared_rank(u[0], rank - 1) : nullptr;
-    T* right = rank + 1 < nc ? cl.map_shared_rank(u[0], rank + 1) : nullptr;
+    T* left = rank > 0 ? cl.map_shared_rank(us, rank - 1) : nullptr;
+    T* right = rank + 1 < nc ? cl.map_shared_rank(us, rank + 1) : nullptr;
     const bool ahead = MODE == kAdj && q.dw && n <= nt && tid < n;
     T dw_next = ahead && q.k0 % q.dw_period == 0
                     ? __ldcs(q.dw + (long long)((q.k0 - q.dw_k0) / q.dw_div) * q.field_stride + sh + a + tid) : T(0);
@@ -155,8 +157,8 @@ __global__ void __launch_bounds__(kThreads1) wave1d_sweep_kernel(const WaveParam
     int cur = 0;
     for (int i = 0; i < q.n; ++i) {
         const int k = q.k0 + q.dir * i;
-        const T *uk = u[cur], *pk = ph[cur];
-        T *un = u[cur ^ 1], *pn = ph[cur ^ 1];
+        const T *uk = us + cur, *pk = ps + cur;
+        T *un = us + (w - cur), *pn = ps + (w - cur);
         if (p.inj.on && i % kAmpSteps == 0) {  // the amplitudes of the next steps
             const T* src = p.inj.amp + (long long)shot * p.inj.amp_sstride;
             const int m = min(kAmpSteps, q.n - i) * q.npts;
@@ -180,8 +182,8 @@ __global__ void __launch_bounds__(kThreads1) wave1d_sweep_kernel(const WaveParam
             auto sample = [&](int e, T& wt, T& v) {
                 const int cell = (int)(__ldg(p.rec.off + e) - kOZ), b = __umulhi(cell, q.inv);
                 wt = __ldg(p.rec.w + e);
-                const T* ub = b == rank ? u[0] : cl.map_shared_rank(u[0], b);
-                v = ub[(uk - u[0]) + cell - b * q.cells];
+                const T* ub = b == rank ? us : cl.map_shared_rank(us, b);
+                v = ub[cur + cell - b * q.cells];
             };
             T* out = q.traces + (long long)shot * p.rec.tr_sstride + (long long)k * p.rec.nrec;
             const int* row = p.rec.rowptr + (long long)shot * p.rec.nrec;
@@ -252,7 +254,7 @@ __global__ void __launch_bounds__(kThreads1) wave1d_sweep_kernel(const WaveParam
             }
             un[j] = unew;
             pn[j] = pnew;
-            const int at = (int)(un - u[0]) + j, pt = (int)(pn - u[0]) + j;
+            const int at = w - cur + j, pt = at + 2 * w;
             if (left && j < R) {
                 left[at + nl] = unew;
                 left[pt + nl] = pnew;
@@ -268,13 +270,13 @@ __global__ void __launch_bounds__(kThreads1) wave1d_sweep_kernel(const WaveParam
             if (MODE == kAdj && img) ic[j] += uc * dw;
         }
         cl.sync();  // the new fields and halos are complete, the old ones free
-        cur ^= 1;
+        cur = w - cur;
         dw_next = dw_after;
     }
     for (int j = tid; j < n; j += blockDim.x) {
-        q.out_cur[sh + a + j] = u[cur][j];
-        q.out_prev[sh + a + j] = u[cur ^ 1][j];
-        q.out_phz[sh + a + j] = ph[cur][j];
+        q.out_cur[sh + a + j] = us[cur + j];
+        q.out_prev[sh + a + j] = us[w - cur + j];
+        q.out_phz[sh + a + j] = ps[cur + j];
         if (MODE == kAdj) p.ic[sh + a + j] = ic[j];
     }
 }
