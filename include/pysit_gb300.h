@@ -292,12 +292,14 @@ int pysit_plan_autotune_tiles(pysit_plan* plan, const int* cand_x, int ncx, cons
 int pysit_plan_get_tiles(const pysit_plan* plan, int* tile_x, int* tile_z);
 /* A host copy of the plan's current task table, no counterpart in the reference (diagnostics
  * and tests; needs no device).  2D: rows of 5 ints (x0, x1, zs, ze, kind: 0 interior, 1 PML
- * shell), the tiles of one shot; 3D: rows of 6 ints (x0, x1, y0, y1, zs, ze), one block of
- * 8 warps at most each, a warp taking 32 / ceil((ze - zs) / V) y-rows (V = 4 FP32, 2 FP64 cells a lane);
- * 1D: none.  The interior tasks come first, *n_interior of them.  *n_ints receives the table's
+ * shell), the tiles of one shot; 3D: rows of 6 ints (x0, x1, y0, y1, zs, ze), one block
+ * each, a warp taking 32 / ceil((ze - zs) / V) y-rows (V = 4 FP32, 2 FP64 cells a lane); 1D: none.  The interior tasks come first, *n_interior of them.  *n_ints receives the table's
  * size in ints; at most cap ints are written to out (which may be NULL). */
 int pysit_plan_task_table(const pysit_plan* plan, int32_t* out, uint64_t cap, uint64_t* n_ints,
                           int32_t* n_interior);
+/* The blocks that step the plan's tiles (diagnostics and tests; needs no device): threads of a block,
+ * and x-rows per thread (2D) or x-planes per thread and round (3D).  0 in 1D. */
+int pysit_plan_get_blocks(const pysit_plan* plan, int* threads, int* rows);
 /* The plan's current tuning: task length along x and the three 2D shell block shares
  * (pysit_plan_desc.shell_share).  Either output may be NULL. */
 int pysit_plan_get_tuning(const pysit_plan* plan, int* tile_x, double* shell_share);

@@ -289,6 +289,7 @@ struct pysit_plan {
     virtual int tiles(int* tile_x, int* tile_z) const = 0;
     // host copy of the current task table (interior tasks first)
     virtual int task_table(int32_t* out, uint64_t cap, uint64_t* n_ints, int32_t* n_interior) const = 0;
+    virtual int blocks(int* threads, int* rows) const = 0;
     // enqueue misfit + gradient on s without graph handling (for a group's capture)
     virtual int enqueue_grad_raw(const void* dobs, double* grad, double* rnorm2, cudaStream_t s) = 0;
     // linearised modelling / Gauss-Newton Hessian application for a model perturbation
@@ -1594,6 +1595,12 @@ struct PlanT final : public pysit_plan {
         return PYSIT_OK;
     }
 
+    int blocks(int* threads, int* rows) const override {
+        if (threads) *threads = dim == 3 ? threads3d : dim == 2 ? threads2d : 0;
+        if (rows) *rows = dim == 3 ? planes3d : dim == 2 ? strip2d : 0;
+        return PYSIT_OK;
+    }
+
     int tuning(int* tile, double* share) const override {
         if (tile) *tile = tx;
         if (share)
@@ -2067,6 +2074,7 @@ struct LanesPlan final : public pysit_plan {
     int task_table(int32_t* out, uint64_t cap, uint64_t* n_ints, int32_t* n_interior) const override {
         return kids[0]->task_table(out, cap, n_ints, n_interior);
     }
+    int blocks(int* threads, int* rows) const override { return kids[0]->blocks(threads, rows); }
 };
 
 }  // namespace
@@ -2217,6 +2225,11 @@ extern "C" int pysit_plan_task_table(const pysit_plan* p, int32_t* out, uint64_t
     PGB_REQUIRE(p, "NULL plan");
     return p->task_table(out, cap, n_ints, n_interior);
 } PGB_API_CATCH("pysit_plan_task_table")
+
+extern "C" int pysit_plan_get_blocks(const pysit_plan* p, int* threads, int* rows) try {
+    PGB_REQUIRE(p, "NULL plan");
+    return p->blocks(threads, rows);
+} PGB_API_CATCH("pysit_plan_get_blocks")
 
 // ---- plan groups ------------------------------------------------------------------------
 struct pysit_group {
