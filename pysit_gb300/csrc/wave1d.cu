@@ -361,8 +361,8 @@ int wave1d_prepare(int nz, int nsrc, int nrec) {
         if (h.nc > 0 && sweep1d_placed<T, R, kFwd>(h, nsrc, sweep1d_recorders(h, nrec)) &&
             sweep1d_placed<T, R, kRecomp>(h, nsrc, sweep1d_recorders(h, nrec)) && sweep1d_placed<T, R, kAdj>(h, nrec, 0))
             return most_nc;
+        cudaGetLastError();  // an attribute or shape that the device refuses is no error of the plan
     }
-    cudaGetLastError();  // an attribute or shape that the device refuses is no error of the plan
     return 0;
 }
 

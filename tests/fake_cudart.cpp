@@ -14,6 +14,7 @@ std::string log_;
 std::map<const void*, std::string> names_;
 struct Config { dim3 grid, block; size_t smem; cudaStream_t stream; } cfg_;
 long next_ = 1;
+cudaError_t last_ = cudaSuccess;
 
 template <typename... A>
 void say(const char* f, A... a) {
@@ -69,7 +70,11 @@ cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void*, const cudaLaunch
     say("query cluster %u", cluster);
     return cudaSuccess;
 }
-cudaError_t cudaFuncSetAttribute(const void*, enum cudaFuncAttribute, int) { return cudaSuccess; }
+// FAKE_PORTABLE: the device takes no clusters of more than eight blocks
+cudaError_t cudaFuncSetAttribute(const void*, enum cudaFuncAttribute a, int) {
+    return a == cudaFuncAttributeNonPortableClusterSizeAllowed && getenv("FAKE_PORTABLE") ? last_ = cudaErrorInvalidValue
+                                                                                         : cudaSuccess;
+}
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = (cudaStream_t)(1000 + next_++); return cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) { say("sync %ld", (long)s); return cudaSuccess; }
@@ -104,7 +109,11 @@ cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t st) {
 }
 cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError() {
+    const cudaError_t e = last_;
+    last_ = cudaSuccess;
+    return e;
+}
 const char* cudaGetErrorName(cudaError_t) { return "fake"; }
 const char* cudaGetErrorString(cudaError_t) { return "fake"; }
 cudaError_t cudaGetSymbolAddress(void**, const void*) { return cudaErrorNotSupported; }

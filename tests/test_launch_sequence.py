@@ -138,3 +138,13 @@ def test_1d_launches_that_fill_the_gpu_step_one_launch_at_a_time(fake, nshots, d
                      "print('\\n'.join(log()))")
     assert sum("wave1d_sweep_kernel" in l for l in out) == runs
     assert sum("wave1d_kernel" in l for l in out) == (0 if runs else 8)
+
+
+@pytest.mark.parametrize("nz,cluster", [(1200, 8), (1500, 0)])
+def test_a_refused_cluster_attribute_is_no_error_of_the_plan(fake, nz, cluster):
+    out = _run(fake, f"d = _desc(keep, 1, (1, 1, {nz}), ((0, 0), (0, 0), (9, 9)), 4, _native.PYSIT_F64)\n"
+                     "h = plan(d); model(h, d); fake.fake_clear()\n"
+                     "tr = np.zeros(8)\n"
+                     "_native.check(lib.pysit_plan_forward(h, C.c_void_p(tr.ctypes.data), C.c_void_p(7)))\n"
+                     "print('\\n'.join(log()))", FAKE_PORTABLE="1")
+    assert [int(l.split()[-1]) for l in out if "wave1d_sweep_kernel" in l] == ([cluster] if cluster else [])
