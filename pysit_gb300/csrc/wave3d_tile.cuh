@@ -19,14 +19,15 @@
 // the outputs through products of two or three sigmas, so the batched path
 // integrates it only where at least two axes are inside the padding.
 //
-// What bounds it: latency (long-scoreboard stalls with four 4-warp blocks per SM at 128 registers;
-// DRAM and L1 below 60 % busy).  Four planes per round need 13 vector loads of u_k per output
-// vector instead of 21, the faces' update 135-180 thread instructions per cell instead of the
-// general update's 276.  Measured against the kernels this one replaces, which walked 64 planes
-// one at a time in two kernels (us per step, before -> now): 440 x 440 x 340, order 8, FP32
-// forward / recompute / adjoint 593 / 595 / 707 -> 491 / 551 / 671; 121 x 107 x 95, order 4, FP32,
-// 4 shots 200 -> 80; 180 x 170 x 150, order 8, FP32 201 -> 56; 53 x 49 x 45, order 4, FP64, 2 shots
-// 708 -> 49.  Three blocks per SM (80 registers, spills) were 12 % slower.
+// What bounds it: latency (two thirds of a warp's cycles wait on loads with four 4-warp blocks per SM at
+// 128 registers; issue slots 27-30 %, DRAM 43-54 %, L1 42-46 % busy; the four-plane kernels of orders 6
+// and 8 spill 4 to 68 bytes in FP32).  Four planes per round need 13 vector loads of u_k per output vector
+// instead of 21, the faces' update 135-180 thread instructions per cell instead of the general update's
+// 276.  Measured against the kernels this one replaces, which walked 64 planes one at a time in two
+// kernels (us per step, before -> now): 440 x 440 x 340, order 8, FP32 forward / recompute / adjoint
+// 593 / 595 / 707 -> 491 / 551 / 671; 121 x 107 x 95, order 4, FP32, 4 shots 200 -> 80; 180 x 170 x 150,
+// order 8, FP32 201 -> 57; 53 x 49 x 45, order 4, FP64, 2 shots 708 -> 49.  Three blocks per SM (80
+// registers, spills) were 12 % slower.
 #pragma once
 #include "pairs.cuh"
 #include "tma.cuh"
@@ -766,8 +767,13 @@ __device__ __forceinline__ void face_planes(const WaveParams<T>& p, const T* rhs
 #ifndef PGB_T3_MINB
 #define PGB_T3_MINB 4  // resident 4-warp blocks per SM the FP32 register budget aims at (128 registers)
 #endif
+// Blocks of 64 threads walk one plane.  At order 8 in FP32 they have 168 registers: at the 128 of the
+// others they spill (50 x 46 x 42 + 6 cells: 60 steps 0.47 ms, 0.45 without spills; order 4, which does not
+// spill, is 7 % slower with 168).
+template <typename T, int R, int RX>
+constexpr int t3_min_blocks() { return sizeof(T) == 8 ? 1 : RX > 1 ? PGB_T3_MINB : R == 4 ? 6 : 2 * PGB_T3_MINB; }
 template <typename T, int R, int MODE, int RX>
-__global__ void __launch_bounds__(kT3, (sizeof(T) == 4 ? PGB_T3_MINB : 1))
+__global__ void __launch_bounds__(RX == 1 ? 64 : kT3, (t3_min_blocks<T, R, RX>()))
     wave3d_tile_kernel(const __grid_constant__ WaveParams<T> p, const Tile3d* __restrict__ tiles, int nint, int nshell,
                        int rec) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
