@@ -48,7 +48,7 @@ METRIC = "FWI gradient shots/s, batched adjoint vs plain, 1\u00d7GB300 at \u2264
 # from one ncu capture of the three step modes at 22 shots per launch
 # (profiles/wave2d_steps_cfg2_22shots_dram.md); a launch's traffic is this times its shots (the
 # kernels' traffic grows in proportion to the shots).
-TRAFFIC_PER_SHOT = {"forward": 195.2e6 / 22, "recompute": 223.1e6 / 22, "adjoint": 345.1e6 / 22}
+TRAFFIC_PER_SHOT = {"forward": 195.1e6 / 22, "recompute": 223.8e6 / 22, "adjoint": 345.5e6 / 22}
 
 
 def max_over_ranks(values, device):
@@ -509,7 +509,7 @@ def main():
             "gpu_launches": launches, "misfit_rnorm2": rn, "clocks": clocks,
             "autotune": {"tile_x": tuned_grad["chosen"], "tile_z": tuned_grad["chosen_z"],
                          "ms": {str(k): v for k, v in tuned_grad["ms"].items()},
-                         "shell_share": tuned_grad.get("shell_share"), "forward_plan_tile_x": tuned["chosen"]}}
+                         "forward_plan_tile_x": tuned["chosen"]}}
     if rank == 0 and not args.no_plain:
         plain = plain_fp64_baseline(scale=args.scale, nsteps_full=args.nsteps)
         plain["batched_over_plain"] = line["value"] / world / plain["value"]

@@ -152,9 +152,9 @@ typedef struct {
     int psi_consistent;            /* 3D PML: 0 = the reference's step, which multiplies sigma_x sigma_y
                                       sigma_z psi by C^2 (_3D.h:219; unstable at realistic PML amplitudes);
                                       1 = that term without C^2, as in the reference's matrix operator */
-    int tile_x;                    /* 2D/3D task length along x in rows at most; 0 = the default (32 in 2D;
-                                      in 3D 1 to 16, by the cells of a launch); pysit_plan_autotune
-                                      chooses it by timing */
+    int tile_x;                    /* 2D/3D task length along x in rows at most; 0 = the default (32 in 2D,
+                                      where a block's rows are the limit; in 3D 1 to 16, by the cells of a
+                                      launch); pysit_plan_autotune chooses it by timing */
     const int32_t* shot_nsteps;    /* host [nshots] or NULL: the record length of each shot in steps
                                       (1..nsteps); the residual of a shot is zero from its length on, so
                                       its misfit and gradient are those of a run of that many steps */

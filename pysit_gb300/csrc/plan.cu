@@ -84,7 +84,7 @@ __global__ void set_c2_kernel(const double* __restrict__ C, int nx, int ny, int 
 // linear in rhs, so adding it afterwards equals injecting it inside the stencil.  One thread per
 // (shot, cell of the shot's injection box); cells of the outer ring are left alone, as the
 // reference skips them.  Used for wide operators (the adjoint source at every receiver), whose
-// per-cell tap walk would stall the stencil's row loop.
+// taps would hold a tile's block back (launch3d).
 template <typename T>
 __global__ void inject_scatter3d_kernel(const WaveParams<T> p, int cells_max) {
     const long long n = (long long)p.nshot * cells_max;
@@ -335,7 +335,7 @@ struct PlanT final : public pysit_plan {
     int threads2d = kT2;         // 2D: threads of a block
     std::vector<Tile2d> tiles2d;      // 2D: the device's form of tasks2d
     int inj_cap[2] = {0, 0};     // 2D, 3D: injection cells of a tile at most (source, receivers)
-    double shell_frac[4] = {0.0, 0.0, 0.0, 0.0};  // descriptor's shell shares (read back by tuning(); unused)
+    double shell_frac[4] = {0.0, 0.0, 0.0, 0.0};  // descriptor's shell shares: read back by tuning(), no effect
     // ---- acquisition (host) ----------------------------------------------------
     std::vector<CSRBox> src_inj, rec_inj;
     int rec_box_max = 0;              // 3D: largest receiver injection box (cells) over the shots
@@ -1067,14 +1067,16 @@ struct PlanT final : public pysit_plan {
         }
     }
 
-    // One 2D step: one launch over the tiles of every shot (the traces recorded and the
-    // injection worked out by the blocks' producer warps).
+    // One 2D step: one launch over the tiles of every shot.  Its leading blocks record the traces; a
+    // tile's block works out the injection of its cells before their update.
     template <int RR, int MODE>
     void launch2d(const WaveParams<T>& p, cudaStream_t s) {
         WaveParams<T> q = p;
-        // a launch whose wavefields exceed L2 (126 MB): a block fetches the next shot's tile.
-        // 64 shots of 1232 x 464 cells (FP32): recompute 175 -> 162, adjoint 248 -> 215 us; two or
-        // three shots ahead 162 / 166 and 230 / 257 us
+        // From 48 MB of wavefields (two fields; Phi, C^2 and a step's outputs fill the rest of L2) a block
+        // fetches the next shot's tile.  1232 x 464 cells, FP32, forward / recompute / adjoint us without and
+        // with it: 64 shots (291 MB) 170 / 187 / 242 and 157 / 166 / 222, 16 shots (73 MB) 44.5 / 49.7 / 63.3
+        // and 43.3 / 45.8 / 60.0, 12 shots (54 MB) 32.4 / 36.9 / 48.1 and 33.0 / 36.1 / 46.9, 8 shots (36 MB)
+        // 18.6 / 21.0 / 31.8 and 20.6 / 22.4 / 33.0.  FP64 is equal within 0.5 %.
         q.pf_next = p.nshot > 1 && 2 * (size_t)fstride * sizeof(T) * p.nshot > ((size_t)48 << 20);
         launch_wave2d_tiles<T, RR, MODE>(q, at<Tile2d>(off.tasks), ntask2d[0], ntask2d[1], strip2d, threads2d,
                                          inj_cap[MODE == kAdj], s);

@@ -21,8 +21,9 @@
 // per row.  Everything is read straight from global memory: the threads of a block share rows
 // and vectors through L1, and a thread's loads are all independent, so four 4-warp blocks per SM
 // (128 registers) keep the memory busy without shared-memory staging, barriers or waits.  What
-// bounds a full launch is latency (long-scoreboard stalls, issue slots 40-45 % busy); a block
-// fetches the same tile of the next shot into L2, whose block starts about when it ends.
+// bounds a full launch is latency (16 warps per SM, long-scoreboard stalls first, issue slots 38-43 %,
+// DRAM 41-53 %, L1 38-44 % busy); a block fetches the same tile of the next shot into L2, whose block
+// starts about when it ends.
 // The injection of a tile's cells (source taps; adjoint source at the receivers) is worked out
 // by the whole block into shared memory before the update, in tiles that meet the shot's box.
 // Tile kinds (block-uniform):

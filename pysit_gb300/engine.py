@@ -27,9 +27,9 @@ __all__ = ["WavePlan", "PlanGroup", "padded_cells", "default_checkpoint_every"]
 
 _DESC_AXIS = {1: [2], 2: [0, 2], 3: [0, 1, 2]}  # mesh axis -> (x, y, z) slot of the descriptor
 
-# tunings chosen by WavePlan.autotune (task length along x, 2D shell block shares per step
-# mode, z extent of the interior tasks), per (kernels, dim, order, padded grid, dtype, psi form, shots per launch, schedule, forward
-# only, lanes); later plans of the same configuration start from them.  With the environment
+# tunings chosen by WavePlan.autotune (task length along x, three numbers of an earlier step of two
+# kernels, kept in the rows and without effect, z extent of the interior tasks), per (kernels, dim,
+# order, padded grid, dtype, psi form, shots per launch, schedule, forward only, lanes); later plans of the same configuration start from them.  With the environment
 # variable PYSIT_CUDA_TUNE_CACHE naming a JSON file, the table is read from that file on first
 # use and written back after every new tuning, so later processes on the machine start from it.
 _TUNED = {}
