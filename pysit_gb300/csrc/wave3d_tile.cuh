@@ -20,13 +20,13 @@
 // integrates it only where at least two axes are inside the padding.
 //
 // What bounds it: latency (two thirds of a warp's cycles wait on loads with four 4-warp blocks per SM at
-// 128 registers; issue slots 27-30 %, DRAM 43-54 %, L1 42-46 % busy; the four-plane kernels of orders 6
-// and 8 spill 4 to 68 bytes in FP32).  Four planes per round need 13 vector loads of u_k per output vector
+// 128 registers; issue slots 28-31 %, DRAM 43-55 %, L1 43-47 % busy; the four-plane kernels of order
+// 8 spill 12 to 60 bytes in FP32).  Four planes per round need 13 vector loads of u_k per output vector
 // instead of 21, the faces' update 135-180 thread instructions per cell instead of the general update's
 // 276.  Measured against the kernels this one replaces, which walked 64 planes one at a time in two
 // kernels (us per step, before -> now): 440 x 440 x 340, order 8, FP32 forward / recompute / adjoint
-// 593 / 595 / 707 -> 491 / 551 / 671; 121 x 107 x 95, order 4, FP32, 4 shots 200 -> 80; 180 x 170 x 150,
-// order 8, FP32 201 -> 57; 53 x 49 x 45, order 4, FP64, 2 shots 708 -> 49.  Three blocks per SM (80
+// 593 / 595 / 707 -> 483 / 530 / 632; 121 x 107 x 95, order 4, FP32, 4 shots 200 -> 80; 180 x 170 x 150,
+// order 8, FP32 201 -> 55; 53 x 49 x 45, order 4, FP64, 2 shots 708 -> 49.  Three blocks per SM (80
 // registers, spills) were 12 % slower.
 #pragma once
 #include "pairs.cuh"
@@ -457,8 +457,8 @@ __device__ __forceinline__ void interior_planes(const WaveParams<T>& p, const T*
             }
     }
     // The other operands of plane r.  The adjoint step reads them before plane r - 1 is stored (440 x
-    // 440 x 340, order 8, FP32: 671 us, 694 after its stores); the other modes, which hold fewer
-    // operands a plane, after (forward 491 us, 498 before).
+    // 440 x 340, order 8, FP32: 3 % faster than after its stores); the other modes, which hold fewer
+    // operands a plane, after (forward 1.5 % faster than before).
     constexpr bool AHEAD = MODE == kAdj;
     Window<T, NP, NB> w;
     Pairs<T, NP> ya[2 * R], cc, um, dwi, ici;
@@ -602,6 +602,11 @@ __device__ __forceinline__ void face_planes(const WaveParams<T>& p, const T* rhs
         }
         ldr(cc, p.c2 + o);
         ldp(um, p.u_prev + sh + o);
+        Pairs<T, NP> dwi, ici;
+        if (MODE == kAdj && p.image) {
+            ldp(dwi, p.dw_in + sh + o);
+            ldp(ici, p.ic + sh + o);
+        }
         P F[NP], duy[NP], duz[NP], uc[NP];
         {
 #pragma unroll
@@ -664,7 +669,7 @@ __device__ __forceinline__ void face_planes(const WaveParams<T>& p, const T* rhs
 #pragma unroll
                 for (int k = 0; k < NP; ++k) F[k] = O::add(F[k], O::mk(rh[2 * k], rh[2 * k + 1]));
         }
-        Pairs<T, NP> un, dwo, nx_, ny_, nz_, dwi, ici;
+        Pairs<T, NP> un, dwo;
         const T s1 = AX == 0 ? sx : col.sy;  // the face's sigma where it is the same for the vector
         const bool pml = AX == 2 ? col.any_sz : s1 != T(0);
         const bool ring = !(col.zall && i > 0 && i < p.nx - 1);
@@ -681,7 +686,7 @@ __device__ __forceinline__ void face_planes(const WaveParams<T>& p, const T* rhs
             un.p[k] = plain[k];
         }
         if (pml) {
-            Pairs<T, NP> phx, phy, phz;
+            Pairs<T, NP> phx, phy, phz, nx_, ny_, nz_;
             ldp(phx, p.phx_in + sh + o);
             ldp(phy, p.phy_in + sh + o);
             const T f1 = AX == 0 ? __ldg(p.fcx + i) : AX == 1 ? __ldg(p.fcy + j) : T(0);
@@ -714,6 +719,9 @@ __device__ __forceinline__ void face_planes(const WaveParams<T>& p, const T* rhs
                     nz_.p[k] = mask(nz_.p[k], k);
                 }
             }
+            stp(p.phx_out + sh + o, nx_);
+            stp(p.phy_out + sh + o, ny_);
+            stp(p.phz_out + sh + o, nz_);
         }
         if (ring)
 #pragma unroll
@@ -732,6 +740,7 @@ __device__ __forceinline__ void face_planes(const WaveParams<T>& p, const T* rhs
                 un.p[k] = O::mk(t[0], t[1]);
             }
         }
+        stp(p.u_prev + sh + o, un);
         if (MODE == kRecomp && p.dw_out) {
             // dWaveOp = C^2 F + (sm - s)(u' - u_{k-1})/(2dt)
             const T m1 = AX == 0 ? __ldg(p.mgx + i) : col.my;
@@ -745,19 +754,11 @@ __device__ __forceinline__ void face_planes(const WaveParams<T>& p, const T* rhs
             }
         }
         if (MODE == kAdj && p.image) {
-            ldp(dwi, p.dw_in + sh + o);
-            ldp(ici, p.ic + sh + o);
 #pragma unroll
             for (int k = 0; k < NP; ++k) ici.p[k] = O::fma(uc[k], dwi.p[k], ici.p[k]);
+            stp(p.ic + sh + o, ici);
         }
-        if (pml) {
-            stp(p.phx_out + sh + o, nx_);
-            stp(p.phy_out + sh + o, ny_);
-            stp(p.phz_out + sh + o, nz_);
-        }
-        stp(p.u_prev + sh + o, un);
         if (MODE == kRecomp && p.dw_out) stp_cs(p.dw_out + sh + o, dwo);
-        if (MODE == kAdj && p.image) stp(p.ic + sh + o, ici);
         if (MODE == kFwd || (MODE == kRecomp && p.nan_check))
 #pragma unroll
             for (int k = 0; k < NP; ++k) chk.see(un.p[k]);
@@ -767,13 +768,8 @@ __device__ __forceinline__ void face_planes(const WaveParams<T>& p, const T* rhs
 #ifndef PGB_T3_MINB
 #define PGB_T3_MINB 4  // resident 4-warp blocks per SM the FP32 register budget aims at (128 registers)
 #endif
-// Blocks of 64 threads walk one plane.  At order 8 in FP32 they have 168 registers: at the 128 of the
-// others they spill (50 x 46 x 42 + 6 cells: 60 steps 0.47 ms, 0.45 without spills; order 4, which does not
-// spill, is 7 % slower with 168).
-template <typename T, int R, int RX>
-constexpr int t3_min_blocks() { return sizeof(T) == 8 ? 1 : RX > 1 ? PGB_T3_MINB : R == 4 ? 6 : 2 * PGB_T3_MINB; }
 template <typename T, int R, int MODE, int RX>
-__global__ void __launch_bounds__(RX == 1 ? 64 : kT3, (t3_min_blocks<T, R, RX>()))
+__global__ void __launch_bounds__(kT3, (sizeof(T) == 4 ? PGB_T3_MINB : 1))
     wave3d_tile_kernel(const __grid_constant__ WaveParams<T> p, const Tile3d* __restrict__ tiles, int nint, int nshell,
                        int rec) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
